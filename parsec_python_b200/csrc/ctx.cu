@@ -3,6 +3,7 @@
 #include "psc_internal.cuh"
 #include "../../include/psc.h"
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <mutex>
@@ -82,6 +83,8 @@ extern "C" int psc_ctx_create(int nx, int ny, int nz, double h, int fd_order, ps
   if ((e = psc_dmalloc(&ctx->red_partial, (size_t)PSC_RED_SLOTS * PSC_RED_BLOCKS * sizeof(double))) !=
       cudaSuccess)
     return fail(e, "partials");
+  if ((e = psc_dmalloc(&ctx->red_ticket, sizeof(unsigned int))) != cudaSuccess) return fail(e, "ticket");
+  if ((e = cudaMemset(ctx->red_ticket, 0, sizeof(unsigned int))) != cudaSuccess) return fail(e, "ticket");
   if ((e = psc_dmalloc(&ctx->scalars, 256 * sizeof(double))) != cudaSuccess) return fail(e, "scalars");
   if ((e = cudaMemset(ctx->scalars, 0, 256 * sizeof(double))) != cudaSuccess) return fail(e, "scalars");
   if ((e = cudaMallocHost(&ctx->host_scalars, 256 * sizeof(double))) != cudaSuccess)
@@ -111,7 +114,7 @@ extern "C" int psc_ctx_destroy(psc_ctx* ctx) {
   for (auto& s : ctx->species) free_species(s);
   psc_free_projectors(ctx);
   psc_dfree(ctx->pot64); psc_dfree(ctx->pot32); psc_dfree(ctx->cheb_coef); psc_dfree(ctx->red_partial);
-  psc_dfree(ctx->scalars); cudaFreeHost(ctx->host_scalars); psc_dfree(ctx->dev_status);
+  psc_dfree(ctx->red_ticket); psc_dfree(ctx->scalars); cudaFreeHost(ctx->host_scalars); psc_dfree(ctx->dev_status);
   psc_dfree(ctx->gram); psc_dfree(ctx->gram2); psc_dfree(ctx->evec); psc_dfree(ctx->tri);
   psc_dfree(ctx->gram_partial); psc_dfree(ctx->lz_v); psc_dfree(ctx->cg_r); psc_dfree(ctx->cg_p);
   psc_dfree(ctx->cg_ap); psc_dfree(ctx->cg_part); psc_dfree(ctx->mix_dx); psc_dfree(ctx->mix_df);
@@ -253,7 +256,8 @@ struct dot_args {
 };
 
 template <int NT>
-__global__ void __launch_bounds__(NT) k_dots_partial(dot_args args, int nslots, long n, double* partial) {
+__global__ void __launch_bounds__(NT)
+k_dots(dot_args args, int nslots, long n, double* partial, unsigned int* ticket, double* __restrict__ out) {
   __shared__ double sh[NT / 32];
   const long chunk = (n + gridDim.x - 1) / gridDim.x;
   const long lo = chunk * blockIdx.x;
@@ -266,16 +270,10 @@ __global__ void __launch_bounds__(NT) k_dots_partial(dot_args args, int nslots, 
     acc = psc_block_sum<double, NT>(acc, sh);
     if (threadIdx.x == 0) partial[(long)s * PSC_RED_BLOCKS + blockIdx.x] = acc;
   }
-}
-
-template <int NT>
-__global__ void __launch_bounds__(NT) k_dots_final(const double* partial, int nslots, double* out) {
-  __shared__ double sh[NT / 32];
-  for (int s = 0; s < nslots; ++s) {
-    double acc = 0.0;
-    for (int i = threadIdx.x; i < PSC_RED_BLOCKS; i += NT) acc += partial[(long)s * PSC_RED_BLOCKS + i];
-    acc = psc_block_sum<double, NT>(acc, sh);
-    if (threadIdx.x == 0) out[s] = acc;
+  if (!psc_last_block(ticket)) return;
+  for (int s = threadIdx.x >> 5; s < nslots; s += NT / 32) {
+    const double v = psc_warp_partials(partial + (long)s * PSC_RED_BLOCKS, gridDim.x);
+    if ((threadIdx.x & 31) == 0) out[s] = v;
   }
 }
 
@@ -284,9 +282,10 @@ int psc_dots(psc_ctx* ctx, int nslots, const double* const* a, const double* con
   PSC_REQUIRE(ctx, nslots >= 1 && nslots <= PSC_RED_SLOTS, "psc_dots: bad slot count");
   dot_args args;
   for (int s = 0; s < nslots; ++s) { args.a[s] = a[s]; args.b[s] = b[s]; }
-  k_dots_partial<256><<<PSC_RED_BLOCKS, 256, 0, st>>>(args, nslots, n, ctx->red_partial);
-  PSC_LAUNCH_CHECK(ctx);
-  k_dots_final<256><<<1, 256, 0, st>>>(ctx->red_partial, nslots, out_dev);
+  // one launch: the last CTA to finish sums the partials.  A CTA takes at
+  // least 1024 entries, so short vectors do not pay for idle CTAs.
+  const int nb = (int)std::max<long>(1, std::min<long>(PSC_RED_BLOCKS, (n + 1023) / 1024));
+  k_dots<256><<<nb, 256, 0, st>>>(args, nslots, n, ctx->red_partial, ctx->red_ticket, out_dev);
   PSC_LAUNCH_CHECK(ctx);
   return 0;
 }

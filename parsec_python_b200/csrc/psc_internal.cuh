@@ -95,6 +95,7 @@ struct psc_ctx {
 
   // deterministic reductions
   double* red_partial = nullptr;  // [PSC_RED_SLOTS][PSC_RED_BLOCKS]
+  unsigned int* red_ticket = nullptr;  // arrival counter of the reductions that end in their last CTA
   double* scalars = nullptr;      // general device scalar scratch [256]
   double* host_scalars = nullptr; // pinned host mirror [256]
 
@@ -279,6 +280,55 @@ __device__ __forceinline__ T psc_block_sum(T v, T* sh /* >= NT/32 */) {
   return r;
 }
 
+// Block-wide sums of NV values per thread with two barriers for all of them
+// (psc_block_sum takes two per value); value q is valid in the threads of warp
+// 0.  Each value is combined in psc_block_sum's order.
+template <int NT, int NV>
+__device__ __forceinline__ void psc_block_sums(double (&v)[NV], double* sh /* >= NV * NT/32 */) {
+  constexpr int NW = NT / 32;
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+#pragma unroll
+  for (int q = 0; q < NV; ++q) v[q] = psc_warp_sum(v[q]);
+  __syncthreads();
+  if (l == 0)
+#pragma unroll
+    for (int q = 0; q < NV; ++q) sh[q * NW + w] = v[q];
+  __syncthreads();
+  if (w == 0)
+#pragma unroll
+    for (int q = 0; q < NV; ++q) v[q] = psc_warp_sum(l < NW ? sh[q * NW + l] : 0.0);
+}
+
+// True in every thread of the CTA that is last to get here: the partials that
+// the other CTAs' thread 0 wrote before are then visible (read them with
+// __ldcg).  The last CTA resets the ticket for the stream's next launch.
+__device__ __forceinline__ bool psc_last_block(unsigned int* ticket) {
+  __shared__ unsigned int s_last;
+  if (threadIdx.x == 0) {
+    __threadfence();
+    const unsigned int t = atomicAdd(ticket, 1u);
+    s_last = t == gridDim.x - 1;
+    if (s_last) *ticket = 0u;
+    __threadfence();
+  }
+  __syncthreads();
+  return s_last != 0u;
+}
+
+// Sum of np partials by one warp: lane l adds part[l], part[l + 32], ... in
+// four interleaved accumulators (the loads of a dependent chain would each
+// wait for the L2), then the shuffle tree.
+__device__ __forceinline__ double psc_warp_partials(const double* part, int np) {
+  const int l = threadIdx.x & 31;
+  double s[4] = {0.0, 0.0, 0.0, 0.0};
+  int i = l;
+  for (; i + 96 < np; i += 128)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) s[q] += __ldcg(part + i + 32 * q);
+  for (int q = 0; i < np; i += 32, ++q) s[q & 3] += __ldcg(part + i);
+  return psc_warp_sum((s[0] + s[1]) + (s[2] + s[3]));
+}
+
 // Ceperley-Alder / Perdew-Zunger LDA of one density value r (electrons per
 // bohr^3), V_xc/exc_nspn.py:73-91: returns v_xc (Ry) and adds the point's
 // energy density 0.75 r v_x + r eps_c to e.  Points with r <= 0 give 0.
@@ -288,12 +338,12 @@ __device__ __forceinline__ double psc_lda_point(double r, double& e) {
   const double c1 = 0.0622, c2 = 0.096, c3 = 0.004, c4 = 0.0232, c5 = 0.0192;
   const double third = 1.0 / 3.0;
   const double pi = 3.141592653589793;
-  const double a0 = pow(4.0 / (9.0 * pi), third);
+  const double a0 = 0.52106176119784808;   // (4 / (9 pi))^(1/3)
   const double twovpia0 = 2.0 / (pi * a0);
   const double p75vpi = 0.75 / pi;
   double v = 0.0;
   if (r > 0.0) {
-    const double rs = pow(p75vpi / r, third);
+    const double rs = cbrt(p75vpi / r);   // a third of pow's instructions, and closer to the exact root
     v = -twovpia0 / rs;
     double ec;
     e += 0.75 * r * v;
