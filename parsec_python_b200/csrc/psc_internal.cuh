@@ -193,10 +193,12 @@ struct psc_ctx {
   double* mix_dx = nullptr;      // [cap][n]
   double* mix_df = nullptr;      // [cap][n]
   double* mix_nv = nullptr;      // [n]  (group vector N for group size 1)
-  double* mix_tmp = nullptr;     // [n]
+  double* mix_tmp = nullptr;     // [n] newest iterate difference
+  double* mix_ddf = nullptr;     // [n] newest residual difference
   double* mix_coef = nullptr;    // [3*cap + 8] dot products and scalars
   double* mix_partial = nullptr; // [3*cap + 2][PSC_RED_BLOCKS]
-  double mix_last_fnorm = -1.0;
+  int mix_slot = 0;              // scalars[120 + mix_slot]: |f|^2 of the last accepted call
+  cudaEvent_t mix_ev = nullptr;  // the two norms have reached the host
 
   std::string last_error;
 };

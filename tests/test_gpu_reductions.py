@@ -76,3 +76,22 @@ def test_occupations_by_state_count(n):
     # the bisections take the same steps: equal up to the rounding of exp
     assert abs(float(ef) - ref_ef) <= 1e-12
     assert np.abs(occ.cpu().numpy() - ref_occ).max() <= 1e-9
+
+
+@pytest.mark.parametrize("dims", [(5, 5, 5), (17, 16, 3), (61, 55, 47)])
+def test_mixer_history_groups_and_restart(dims):
+    """Thirteen secant columns (three groups of four and one over), a restart,
+    and four more, against the oracle's msecant1."""
+    ctx = _ctx(dims)
+    rng = np.random.default_rng(sum(dims))
+    ours, ref = gpu.Mixer(ctx, 40), O.MSecant1()
+    for i in range(19):
+        f = rng.standard_normal(ctx.n) * 0.7 ** i
+        if i >= 14:
+            f *= 1e3      # |f| of the call before < 0.1 |f|: restart at i = 14
+        x = 1.0 + 0.5 ** i * rng.standard_normal(ctx.n)
+        got, m = ours(_dev(x), _dev(f))
+        want, m_ref = ref(x, f)
+        assert m == m_ref and (i != 14 or m == 0)
+        # independent columns: the secant equations are well conditioned
+        assert np.abs(got.cpu().numpy() - want).max() <= 1e-10 * np.abs(want).max()
