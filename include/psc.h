@@ -334,12 +334,12 @@ int psc_conv3d_fwd(psc_ctx* ctx, const int* geom, const void* A, const void* S, 
 /* Forward implementation: 2 the tcgen05 implicit GEMM (BF16 operands, FP32
  * accumulation in tensor memory; activations 16-byte aligned), 0 the
  * CUDA-core kernel, 1 (default) by layer: tcgen05 from 32 output channels.
- * The backward always runs on the CUDA cores. */
+ * The backward always runs on the tensor cores (conv_bwd.cu). */
 int psc_set_conv_impl(psc_ctx* ctx, int impl);
 /* act: 0 identity, 1 ReLU, 2 leaky ReLU (slope 1/16 below zero).
  * Backward of one convolution.  gout: dL/d(out) FP32 [nvo][Cout]; out: the
  * forward's BF16 output (needed when act != 0);
- * gm: FP32 scratch [nvo][Cout] (may alias gout); dvin: FP32 scratch
+ * gm: FP32 scratch [nvo][Cout] (may alias gout; contents unspecified); dvin: FP32 scratch
  * [nvi][Ca+Cs] or NULL to skip the input gradient; dA / dS: FP32 gradients of
  * A and S, overwritten (acc = 0) or accumulated (acc = 1), NULL to skip; dW,
  * dB: FP32 weight and bias gradients (overwritten); work: FP32 scratch of

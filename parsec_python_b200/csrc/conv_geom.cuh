@@ -1,6 +1,7 @@
 // Geometry of one 3-D convolution of the learned-start network and the
 // 8-channel gather of its "virtual input" (shared by the CUDA-core kernels in
-// unet.cu and the tensor-core forward in conv_tc.cu).
+// unet.cu and the tensor-core forward and backward in conv_tc.cu and
+// conv_bwd.cu).
 //
 // Activations are channels-last BF16 tensors [voxel][C] on a grid with x
 // fastest (voxel = x + nx (y + ny z)), C a multiple of 8.  The virtual input
@@ -39,3 +40,11 @@ __device__ __forceinline__ uint4 conv_vin8(const __nv_bfloat16* A, const __nv_bf
 int psc_conv_tc_forward(psc_ctx* ctx, const ConvGeom& g, const __nv_bfloat16* a, const __nv_bfloat16* s,
                         const __nv_bfloat16* w, const float* bias, int act, __nv_bfloat16* o, float* out32,
                         cudaStream_t st);
+
+// backward on the tensor cores (conv_bwd.cu): planes of the gradient, dW and
+// dB; then the input gradient (all Cin channels, ldo floats per voxel)
+int psc_conv_bwd_weights(psc_ctx* ctx, const ConvGeom& g, const __nv_bfloat16* a, const __nv_bfloat16* s,
+                         const float* gout, const __nv_bfloat16* out, int act, float* dW, float* dB, float* work,
+                         long work_floats, cudaStream_t st);
+int psc_conv_bwd_input(psc_ctx* ctx, const ConvGeom& g, const __nv_bfloat16* w, float* out, int ldo, int acc,
+                       cudaStream_t st);

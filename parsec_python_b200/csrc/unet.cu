@@ -111,182 +111,6 @@ k_conv_fwd(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict_
   }
 }
 
-// ---------------------------------------------------------------------------
-// backward data: dvin[v][ci] = sum_tap sum_co gm[o(v,tap)][co] W[tap][ci][co]
-// where o s + tap - pad = v.  One thread per virtual-input voxel, CIT input
-// channels per CTA; the output channels are walked in chunks of 256 / CIT.
-// ---------------------------------------------------------------------------
-template <int CIT>
-__global__ void __launch_bounds__(FWD_NT)
-k_conv_bwd_data(const float* __restrict__ gm, const __nv_bfloat16* __restrict__ W, ConvGeom g,
-                float* __restrict__ dvin) {
-  constexpr int COUT_CHUNK = WTILE / CIT;
-  __shared__ __align__(16) float ws[27 * WTILE];
-  const int taps = g.ksize * g.ksize * g.ksize;
-  const int pad = g.ksize / 2;
-  const int ci0 = blockIdx.y * CIT;
-  const long nvi = (long)g.nxi * g.nyi * g.nzi;
-  const long v = (long)blockIdx.x * FWD_NT + threadIdx.x;
-  const bool valid = v < nvi;
-  int x = 0, y = 0, z = 0;
-  if (valid) {
-    x = (int)(v % g.nxi);
-    const long r = v / g.nxi;
-    y = (int)(r % g.nyi);
-    z = (int)(r / g.nyi);
-  }
-  float acc[CIT];
-#pragma unroll
-  for (int j = 0; j < CIT; ++j) acc[j] = 0.0f;
-  for (int oc = 0; oc < g.Cout; oc += COUT_CHUNK) {
-    const int on = min(COUT_CHUNK, g.Cout - oc);
-    __syncthreads();
-    for (int e = threadIdx.x; e < taps * on * CIT; e += FWD_NT) {
-      const int ci = e % CIT;
-      const int r = e / CIT;
-      const int co = r % on, tap = r / on;
-      ws[(tap * COUT_CHUNK + co) * CIT + ci] = __bfloat162float(W[((long)tap * g.Cin + ci0 + ci) * g.Cout + oc + co]);
-    }
-    __syncthreads();
-    if (!valid) continue;
-    for (int tap = 0; tap < taps; ++tap) {
-      const int dx = tap % g.ksize, dy = (tap / g.ksize) % g.ksize, dz = tap / (g.ksize * g.ksize);
-      // o s = v - d + pad
-      const int ax = x - dx + pad, ay = y - dy + pad, az = z - dz + pad;
-      if (ax < 0 || ay < 0 || az < 0) continue;
-      if (g.stride == 2 && ((ax | ay | az) & 1)) continue;
-      const int ox = ax / g.stride, oy = ay / g.stride, oz = az / g.stride;
-      if (ox >= g.nxo || oy >= g.nyo || oz >= g.nzo) continue;
-      const float* gp = gm + (ox + (long)g.nxo * (oy + (long)g.nyo * oz)) * g.Cout + oc;
-      for (int co4 = 0; co4 < on; co4 += 4) {
-        const float4 g4 = *reinterpret_cast<const float4*>(gp + co4);
-        const float gv[4] = {g4.x, g4.y, g4.z, g4.w};
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float* wr = ws + (tap * COUT_CHUNK + co4 + j) * CIT;
-#pragma unroll
-          for (int ci = 0; ci < CIT; ci += 4) {
-            const float4 w4 = *reinterpret_cast<const float4*>(wr + ci);
-            acc[ci] = fmaf(gv[j], w4.x, acc[ci]);
-            acc[ci + 1] = fmaf(gv[j], w4.y, acc[ci + 1]);
-            acc[ci + 2] = fmaf(gv[j], w4.z, acc[ci + 2]);
-            acc[ci + 3] = fmaf(gv[j], w4.w, acc[ci + 3]);
-          }
-        }
-      }
-    }
-  }
-  if (!valid) return;
-#pragma unroll
-  for (int j = 0; j < CIT; ++j) dvin[v * g.Cin + ci0 + j] = acc[j];
-}
-
-// ---------------------------------------------------------------------------
-// backward weights: part[chunk][tap][ci][co] = sum over the chunk's output
-// voxels of vin(o s + tap - pad)[ci] gm[o][co].  A CTA owns one tap, a 16x16
-// (ci, co) tile and one voxel chunk; it stages 64 voxels at a time.
-// ---------------------------------------------------------------------------
-constexpr int BW_NT = 256;
-constexpr int BW_STAGE = 64;
-
-__global__ void __launch_bounds__(BW_NT)
-k_conv_bwd_w(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict__ S,
-             const float* __restrict__ gm, ConvGeom g, int vchunk, float* __restrict__ part) {
-  __shared__ float xs[BW_STAGE][17];
-  __shared__ float gs[BW_STAGE][17];
-  const int taps = g.ksize * g.ksize * g.ksize;
-  const int pad = g.ksize / 2;
-  const int nci = (g.Cin + 15) / 16, nco = (g.Cout + 15) / 16;
-  int t = blockIdx.y;
-  const int cot = t % nco;
-  t /= nco;
-  const int cit = t % nci;
-  const int tap = t / nci;
-  const int ci0 = cit * 16, co0 = cot * 16;
-  const int dx = tap % g.ksize, dy = (tap / g.ksize) % g.ksize, dz = tap / (g.ksize * g.ksize);
-  const long nvo = (long)g.nxo * g.nyo * g.nzo;
-  const long v_begin = (long)blockIdx.x * vchunk;
-  const long v_end = min(nvo, v_begin + vchunk);
-  const int tci = threadIdx.x >> 4, tco = threadIdx.x & 15;
-  float acc = 0.0f;
-  for (long v0 = v_begin; v0 < v_end; v0 += BW_STAGE) {
-    __syncthreads();
-    // stage inputs: 64 voxels x two groups of 8 channels (threads 0..127)
-    if (threadIdx.x < 2 * BW_STAGE) {
-      const int j = threadIdx.x >> 1, half = threadIdx.x & 1;
-      const long vo = v0 + j;
-      const int c0 = ci0 + 8 * half;
-      float x[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-      if (vo < v_end && c0 < g.Cin) {
-        const int xo = (int)(vo % g.nxo);
-        const long r = vo / g.nxo;
-        const int yo = (int)(r % g.nyo), zo = (int)(r / g.nyo);
-        const int xi = xo * g.stride + dx - pad, yi = yo * g.stride + dy - pad, zi = zo * g.stride + dz - pad;
-        if (xi >= 0 && yi >= 0 && zi >= 0 && xi < g.nxi && yi < g.nyi && zi < g.nzi)
-          unpack8(conv_vin8(A, S, g, xi, yi, zi, c0), x);
-      }
-#pragma unroll
-      for (int i = 0; i < 8; ++i) xs[j][8 * half + i] = x[i];
-    } else {
-      // stage gradients: 64 voxels x 16 channels as float4 (threads 128..255, two each)
-      for (int q = threadIdx.x - 2 * BW_STAGE; q < BW_STAGE * 4; q += BW_NT - 2 * BW_STAGE) {
-        const int j = q >> 2, c4 = (q & 3) * 4;
-        const long vo = v0 + j;
-        float4 g4 = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (vo < v_end && co0 + c4 < g.Cout) g4 = *reinterpret_cast<const float4*>(gm + vo * g.Cout + co0 + c4);
-        gs[j][c4] = g4.x;
-        gs[j][c4 + 1] = g4.y;
-        gs[j][c4 + 2] = g4.z;
-        gs[j][c4 + 3] = g4.w;
-      }
-    }
-    __syncthreads();
-#pragma unroll 16
-    for (int j = 0; j < BW_STAGE; ++j) acc = fmaf(xs[j][tci], gs[j][tco], acc);
-  }
-  const int ci = ci0 + tci, co = co0 + tco;
-  if (ci < g.Cin && co < g.Cout) part[(((long)blockIdx.x * taps + tap) * g.Cin + ci) * g.Cout + co] = acc;
-}
-
-// dW[e] = sum_chunk part[chunk][e] in chunk order
-__global__ void k_sum_chunks(const float* __restrict__ part, int nchunk, long nw, float* __restrict__ dW) {
-  for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < nw; e += (long)gridDim.x * blockDim.x) {
-    float s = 0.0f;
-    for (int c = 0; c < nchunk; ++c) s += part[(long)c * nw + e];
-    dW[e] = s;
-  }
-}
-
-// bias gradient partials: per CTA (voxel chunk) and channel, then summed by
-// k_sum_chunks.  256 threads = R rows x Cout channels (Cout <= 256); row r
-// sums voxels v0 + r, v0 + r + R, ...; the rows are combined in order.
-__global__ void __launch_bounds__(256)
-k_bias_partial(const float* __restrict__ gm, long nvo, int Cout, int vchunk, float* __restrict__ part) {
-  __shared__ float sh[256];
-  const long v0 = (long)blockIdx.x * vchunk;
-  const long v1 = min(nvo, v0 + vchunk);
-  const int R = 256 / Cout;
-  const int co = threadIdx.x % Cout, r = threadIdx.x / Cout;
-  float s = 0.0f;
-  if (r < R)
-    for (long v = v0 + r; v < v1; v += R) s += gm[v * Cout + co];
-  sh[threadIdx.x] = s;
-  __syncthreads();
-  if (threadIdx.x < Cout) {
-    float t = 0.0f;
-    for (int q = 0; q < R; ++q) t += sh[q * Cout + threadIdx.x];
-    part[(long)blockIdx.x * Cout + threadIdx.x] = t;
-  }
-}
-
-// gm = g * act'(pre) from the BF16 activation (out > 0 exactly when pre > 0):
-// 1 above zero, 0 (ReLU) or the leak slope (leaky ReLU) below
-__global__ void k_relu_grad(const float* __restrict__ gin, const __nv_bfloat16* __restrict__ out, long n,
-                            float below, float* __restrict__ gm) {
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
-    gm[i] = __bfloat162float(out[i]) > 0.0f ? gin[i] : below * gin[i];
-}
-
 // Split the virtual-input gradient: dA (+)= pool(dvin[:, :Ca]) (sum over the
 // 8 fine voxels of each coarse one when up), dS (+)= dvin[:, Ca:].
 __global__ void k_split_grad_a(const float* __restrict__ dvin, ConvGeom g, int accumulate, float* __restrict__ dA) {
@@ -453,60 +277,25 @@ extern "C" int psc_conv3d_bwd(psc_ctx* ctx, const int* geom, const void* A, cons
   PSC_REQUIRE(ctx, act >= 0 && act <= 2 && (act == 0 || out), "conv3d_bwd: bad activation arguments");
   PSC_REQUIRE(ctx, A && W && gout && gm && dW && dB && work && (g.Cs == 0 || S), "conv3d_bwd: NULL pointer");
   cudaStream_t st = (cudaStream_t)stream;
-  const long nvo = (long)g.nxo * g.nyo * g.nzo;
-  const long nvi = (long)g.nxi * g.nyi * g.nzi;
-  const int taps = g.ksize * g.ksize * g.ksize;
   const auto* a = static_cast<const __nv_bfloat16*>(A);
   const auto* s = static_cast<const __nv_bfloat16*>(S);
   const auto* w = static_cast<const __nv_bfloat16*>(W);
-  // 1. output gradient through the activation
-  if (act != 0) {
-    k_relu_grad<<<148 * 8, 256, 0, st>>>(gout, static_cast<const __nv_bfloat16*>(out), nvo * g.Cout,
-                                         act == 2 ? LEAK : 0.0f, gm);
-    PSC_LAUNCH_CHECK(ctx);
-  } else if (gm != gout) {
-    PSC_CUDA(ctx, cudaMemcpyAsync(gm, gout, nvo * g.Cout * sizeof(float), cudaMemcpyDeviceToDevice, st));
-  }
-  // 2. weight and bias gradients (partials in `work`, summed in chunk order)
-  const long nw = (long)taps * g.Cin * g.Cout;
-  int vchunk = 4096;
-  int nchunk = psc_div_up(nvo, vchunk);
-  while ((long)nchunk * nw > work_floats && vchunk < (1 << 26)) {
-    vchunk *= 2;
-    nchunk = psc_div_up(nvo, vchunk);
-  }
-  PSC_REQUIRE(ctx, (long)nchunk * nw <= work_floats && (long)nchunk * g.Cout <= work_floats,
-              "conv3d_bwd: work buffer too small");
-  {
-    const int nci = (g.Cin + 15) / 16, nco = (g.Cout + 15) / 16;
-    dim3 grid(nchunk, taps * nci * nco);
-    k_conv_bwd_w<<<grid, BW_NT, 0, st>>>(a, s, gm, g, vchunk, work);
-    PSC_LAUNCH_CHECK(ctx);
-    k_sum_chunks<<<psc_div_up(nw, 256), 256, 0, st>>>(work, nchunk, nw, dW);
-    PSC_LAUNCH_CHECK(ctx);
-    k_bias_partial<<<nchunk, 256, 0, st>>>(gm, nvo, g.Cout, vchunk, work);
-    PSC_LAUNCH_CHECK(ctx);
-    k_sum_chunks<<<1, 256, 0, st>>>(work, nchunk, g.Cout, dB);
+  // output gradient through the activation, weight and bias gradients
+  int rc = psc_conv_bwd_weights(ctx, g, a, s, gout, static_cast<const __nv_bfloat16*>(out), act, dW, dB, work,
+                                work_floats, st);
+  if (rc || !dvin) return rc;
+  // input gradient: straight into dA when it is A's alone, else through dvin
+  // and split into dA and dS
+  if (!g.up && g.Cs == 0 && dA) return psc_conv_bwd_input(ctx, g, w, dA, g.Ca, acc_a, st);
+  rc = psc_conv_bwd_input(ctx, g, w, dvin, g.Cin, 0, st);
+  if (rc) return rc;
+  if (dA) {
+    k_split_grad_a<<<148 * 8, 256, 0, st>>>(dvin, g, acc_a, dA);
     PSC_LAUNCH_CHECK(ctx);
   }
-  // 3. input gradient, split into dA and dS
-  if (dvin) {
-    if (g.Cin % 16 == 0) {
-      dim3 grid(psc_div_up(nvi, FWD_NT), g.Cin / 16);
-      k_conv_bwd_data<16><<<grid, FWD_NT, 0, st>>>(gm, w, g, dvin);
-    } else {
-      dim3 grid(psc_div_up(nvi, FWD_NT), g.Cin / 8);
-      k_conv_bwd_data<8><<<grid, FWD_NT, 0, st>>>(gm, w, g, dvin);
-    }
+  if (dS && g.Cs > 0) {
+    k_split_grad_s<<<148 * 8, 256, 0, st>>>(dvin, g, acc_s, dS);
     PSC_LAUNCH_CHECK(ctx);
-    if (dA) {
-      k_split_grad_a<<<148 * 8, 256, 0, st>>>(dvin, g, acc_a, dA);
-      PSC_LAUNCH_CHECK(ctx);
-    }
-    if (dS && g.Cs > 0) {
-      k_split_grad_s<<<148 * 8, 256, 0, st>>>(dvin, g, acc_s, dS);
-      PSC_LAUNCH_CHECK(ctx);
-    }
   }
   return 0;
 }
