@@ -22,6 +22,41 @@ extern "C" const char* psc_last_error(const psc_ctx* ctx) {
   return g_last_error.c_str();
 }
 
+// Pinned host scratch of the contexts (256 doubles each).  Pinning memory
+// takes a millisecond or more, as long as the rest of a context's creation, so
+// up to 16 blocks of destroyed contexts are kept for later ones.  A block has
+// no copy in flight when its context is destroyed: every entry point that
+// copies into it waits for the copy before it returns.
+constexpr size_t PIN_BYTES = 256 * sizeof(double);
+constexpr size_t PIN_KEEP = 16;
+static std::mutex g_pin_mu;
+// (never destroyed: a context may outlive the library's static objects)
+static std::vector<double*>& g_pin_free = *new std::vector<double*>;
+
+static cudaError_t pin_take(double** p) {
+  {
+    std::lock_guard<std::mutex> lk(g_pin_mu);
+    if (!g_pin_free.empty()) {
+      *p = g_pin_free.back();
+      g_pin_free.pop_back();
+      return cudaSuccess;
+    }
+  }
+  return cudaHostAlloc(reinterpret_cast<void**>(p), PIN_BYTES, cudaHostAllocPortable);
+}
+
+static void pin_give(double* p) {
+  if (!p) return;
+  {
+    std::lock_guard<std::mutex> lk(g_pin_mu);
+    if (g_pin_free.size() < PIN_KEEP) {
+      g_pin_free.push_back(p);
+      return;
+    }
+  }
+  cudaFreeHost(p);
+}
+
 extern "C" int psc_version(void) { return PSC_ABI_VERSION; }
 
 // Finite-difference weights of -h^2 d2/dx2 summed over the axes
@@ -87,7 +122,7 @@ extern "C" int psc_ctx_create(int nx, int ny, int nz, double h, int fd_order, ps
   if ((e = cudaMemset(ctx->red_ticket, 0, sizeof(unsigned int))) != cudaSuccess) return fail(e, "ticket");
   if ((e = psc_dmalloc(&ctx->scalars, 256 * sizeof(double))) != cudaSuccess) return fail(e, "scalars");
   if ((e = cudaMemset(ctx->scalars, 0, 256 * sizeof(double))) != cudaSuccess) return fail(e, "scalars");
-  if ((e = cudaMallocHost(&ctx->host_scalars, 256 * sizeof(double))) != cudaSuccess)
+  if ((e = pin_take(&ctx->host_scalars)) != cudaSuccess)
     return fail(e, "host scalars");
   if ((e = psc_dmalloc(&ctx->dev_status, 8 * sizeof(int))) != cudaSuccess) return fail(e, "status");
   if ((e = cudaMemset(ctx->dev_status, 0, 8 * sizeof(int))) != cudaSuccess) return fail(e, "status");
@@ -100,10 +135,9 @@ extern "C" int psc_ctx_create(int nx, int ny, int nz, double h, int fd_order, ps
 }
 
 static void free_species(psc_species& s) {
-  for (int i = 0; i < 5; ++i) {
-    psc_dfree(s.x[i]); psc_dfree(s.z[i]); psc_dfree(s.c[i]); psc_dfree(s.d[i]);
-    s.x[i] = s.z[i] = s.c[i] = s.d[i] = nullptr;
-  }
+  psc_dfree(s.block);
+  s.block = nullptr;
+  for (int i = 0; i < 5; ++i) s.x[i] = s.z[i] = s.c[i] = s.d[i] = nullptr;
   s.valid = 0;
 }
 
@@ -114,7 +148,7 @@ extern "C" int psc_ctx_destroy(psc_ctx* ctx) {
   for (auto& s : ctx->species) free_species(s);
   psc_free_projectors(ctx);
   psc_dfree(ctx->pot64); psc_dfree(ctx->pot32); psc_dfree(ctx->cheb_coef); psc_dfree(ctx->red_partial);
-  psc_dfree(ctx->red_ticket); psc_dfree(ctx->scalars); cudaFreeHost(ctx->host_scalars); psc_dfree(ctx->dev_status);
+  psc_dfree(ctx->red_ticket); psc_dfree(ctx->scalars); pin_give(ctx->host_scalars); psc_dfree(ctx->dev_status);
   psc_dfree(ctx->gram); psc_dfree(ctx->gram2); psc_dfree(ctx->evec); psc_dfree(ctx->tri);
   psc_dfree(ctx->gram_partial); psc_dfree(ctx->lz_v); psc_dfree(ctx->cg_r); psc_dfree(ctx->cg_p);
   psc_dfree(ctx->cg_ap); psc_dfree(ctx->cg_part); psc_dfree(ctx->mix_dx); psc_dfree(ctx->mix_df);
@@ -208,6 +242,9 @@ extern "C" int psc_set_species(psc_ctx* ctx, int species_id, int nknots, const d
     cols[3][i] = row[5];
     cols[4][i] = row[3] - row[4];
   }
+  // the five splines are packed and uploaded at once: x, z (nk each), c, d (nk - 1 each)
+  std::vector<double> pack;
+  size_t off[5][4];
   for (int f = 0; f < 5; ++f) {
     std::vector<int> keep;
     prune_knots(cols[f], keep);
@@ -216,14 +253,19 @@ extern "C" int psc_set_species(psc_ctx* ctx, int species_id, int nknots, const d
     PSC_REQUIRE(ctx, natural_spline(xk, yk, z, c, d) == 0, "spline needs >= 3 distinct knots");
     const int nk = (int)xk.size();
     s.nk[f] = nk;
-    PSC_CUDA(ctx, psc_dmalloc(&s.x[f], nk * sizeof(double)));
-    PSC_CUDA(ctx, psc_dmalloc(&s.z[f], nk * sizeof(double)));
-    PSC_CUDA(ctx, psc_dmalloc(&s.c[f], (nk - 1) * sizeof(double)));
-    PSC_CUDA(ctx, psc_dmalloc(&s.d[f], (nk - 1) * sizeof(double)));
-    PSC_CUDA(ctx, cudaMemcpy(s.x[f], xk.data(), nk * sizeof(double), cudaMemcpyHostToDevice));
-    PSC_CUDA(ctx, cudaMemcpy(s.z[f], z.data(), nk * sizeof(double), cudaMemcpyHostToDevice));
-    PSC_CUDA(ctx, cudaMemcpy(s.c[f], c.data(), (nk - 1) * sizeof(double), cudaMemcpyHostToDevice));
-    PSC_CUDA(ctx, cudaMemcpy(s.d[f], d.data(), (nk - 1) * sizeof(double), cudaMemcpyHostToDevice));
+    const std::vector<double>* part[4] = {&xk, &z, &c, &d};
+    for (int q = 0; q < 4; ++q) {
+      off[f][q] = pack.size();
+      pack.insert(pack.end(), part[q]->begin(), part[q]->begin() + (q < 2 ? nk : nk - 1));
+    }
+  }
+  PSC_CUDA(ctx, psc_dmalloc(&s.block, pack.size() * sizeof(double)));
+  PSC_CUDA(ctx, cudaMemcpy(s.block, pack.data(), pack.size() * sizeof(double), cudaMemcpyHostToDevice));
+  for (int f = 0; f < 5; ++f) {
+    s.x[f] = s.block + off[f][0];
+    s.z[f] = s.block + off[f][1];
+    s.c[f] = s.block + off[f][2];
+    s.d[f] = s.block + off[f][3];
   }
   s.zvalue = zvalue;
   s.rcut = rcut;

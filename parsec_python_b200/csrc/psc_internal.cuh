@@ -29,6 +29,7 @@ struct psc_species {
   // Five natural cubic splines on pruned knots: 0 charge, 1 hartree, 2 pot_S,
   // 3 wfn_P, 4 pot_P - pot_S.  Device arrays x, z, c, d per spline.
   int nk[5] = {0, 0, 0, 0, 0};
+  double* block = nullptr;  // one device allocation; the pointers below lie in it
   double* x[5] = {nullptr};
   double* z[5] = {nullptr};
   double* c[5] = {nullptr};
@@ -77,6 +78,7 @@ struct psc_ctx {
   // projector tables: n_atoms_nl atoms, compacted ball points
   int nl_atoms = 0;
   long nl_points = 0;
+  void* nl_block = nullptr;      // one device allocation; the tables below lie in it
   int* nl_atom_off = nullptr;    // [nl_atoms+1] offsets into the point arrays
   int* nl_idx = nullptr;         // [nl_points] grid index of each ball point
   double* nl_u64 = nullptr;      // [3][nl_points]
