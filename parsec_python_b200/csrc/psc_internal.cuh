@@ -162,11 +162,10 @@ struct psc_ctx {
   };
   std::vector<StencilSched> st_sched;
 
-  // spectral Poisson preconditioner: DST-I matrices (m x mp, mp = m rounded
-  // up to 16), per-axis eigenvalues of the stencil, two work vectors
+  // spectral Poisson preconditioner: half-size DST-I matrices of the even and
+  // odd modes, per-axis eigenvalues of the stencil, one work vector
   double* spec_S[3] = {nullptr, nullptr, nullptr};
   double* spec_lam[3] = {nullptr, nullptr, nullptr};
-  int spec_mp[3] = {0, 0, 0};
   double* spec_tmp = nullptr;
 
   // Lanczos vectors (double)
@@ -392,7 +391,7 @@ int psc_tridiag_eig_impl(psc_ctx* ctx, const double* ab, int k, int nvec, double
                          double crel, cudaStream_t st);
 int psc_stencil_blocks(psc_ctx* ctx, int k);
 int psc_laplacian_fused(psc_ctx* ctx, const double* x, const double* prev, double* y, double a, double b,
-                        double g, double* dot_partial, int* nblocks, cudaStream_t st);
+                        double g, double* dot_partial, int* nblocks, cudaStream_t st, const double* active = nullptr);
 int psc_random_impl(psc_ctx* ctx, int dtype, int dist, unsigned long long seed, void* out, long ld,
                     long rows, int cols, cudaStream_t st);
 // zero the points outside the sphere mask in k columns (no-op without a mask)

@@ -27,7 +27,8 @@ __global__ void __launch_bounds__(256)
 k_stencil(const T* __restrict__ X, long ldx, const T* Pv, long ldp, T* Y, long ldy,
           const T* __restrict__ pot, int nx, int ny, int nz, int zchunk, StencilW<T> w,
           const double* __restrict__ coef, double ha, double hb, double hg,
-          double* __restrict__ dot_partial) {
+          double* __restrict__ dot_partial, const double* __restrict__ active) {
+  if (active && *active == 0.0) return;   // a solver's launch past its convergence
   constexpr int NT = 256;
   constexpr int S = NT * PPT;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -153,13 +154,14 @@ static StencilPlan plan_stencil(const psc_ctx* ctx, int k, size_t elem) {
 template <typename T, int R, int PPT>
 static int launch_stencil_t(psc_ctx* ctx, const StencilPlan& p, const T* X, long ldx, const T* P,
                             long ldp, T* Y, long ldy, const T* pot, StencilW<T> w, const double* coef,
-                            double a, double b, double g, double* dot_partial, cudaStream_t st) {
+                            double a, double b, double g, double* dot_partial, const double* active,
+                            cudaStream_t st) {
   auto kern = k_stencil<T, R, PPT>;
   if (p.smem > 40 * 1024) {
     PSC_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem));
   }
   kern<<<p.grid, 256, p.smem, st>>>(X, ldx, P, ldp, Y, ldy, pot, ctx->nx, ctx->ny, ctx->nz, p.zchunk, w,
-                                    coef, a, b, g, dot_partial);
+                                    coef, a, b, g, dot_partial, active);
   PSC_LAUNCH_CHECK(ctx);
   return 0;
 }
@@ -200,7 +202,8 @@ int psc_mask_block_impl(psc_ctx* ctx, int dtype, void* X, long ld, int k, cudaSt
 template <typename T>
 static int launch_stencil(psc_ctx* ctx, int k, const T* X, long ldx, const T* P, long ldp, T* Y, long ldy,
                           const T* pot, const double* c0c, const double* coef, double a, double b,
-                          double g, double* dot_partial, int* nblocks_out, cudaStream_t st, bool masked = false) {
+                          double g, double* dot_partial, int* nblocks_out, cudaStream_t st, bool masked = false,
+                          const double* active = nullptr) {
   // the TMA pipeline serves every launch that needs no fused dot product and
   // meets the bulk-copy alignment rules; the register-queue kernel the rest
   // (followed by a masking pass when the Hamiltonian is sphere-masked)
@@ -224,9 +227,9 @@ static int launch_stencil(psc_ctx* ctx, int k, const T* X, long ldx, const T* P,
   if (R == RR) {                                                                                   \
     if (p.ppt == 2)                                                                                \
       return launch_stencil_t<T, RR, 2>(ctx, p, X, ldx, P, ldp, Y, ldy, pot, w, coef, a, b, g,     \
-                                        dot_partial, st);                                         \
+                                        dot_partial, active, st);                                 \
     return launch_stencil_t<T, RR, 1>(ctx, p, X, ldx, P, ldp, Y, ldy, pot, w, coef, a, b, g,       \
-                                      dot_partial, st);                                           \
+                                      dot_partial, active, st);                                   \
   }
   PSC_DISPATCH(1) PSC_DISPATCH(2) PSC_DISPATCH(3) PSC_DISPATCH(4)
 #undef PSC_DISPATCH
@@ -238,12 +241,13 @@ int psc_stencil_blocks(psc_ctx* ctx, int k) {
   return (int)(p.grid.x * p.grid.y * p.grid.z);
 }
 
-// Laplacian (k = 1, double) with an optional fused per-block partial of Out.In.
+// Laplacian (k = 1, double) with an optional fused per-block partial of Out.In;
+// with a partial, `active` (device, may be NULL) = 0 makes the launch do nothing.
 int psc_laplacian_fused(psc_ctx* ctx, const double* x, const double* prev, double* y, double a, double b,
-                        double g, double* dot_partial, int* nblocks, cudaStream_t st) {
+                        double g, double* dot_partial, int* nblocks, cudaStream_t st, const double* active) {
   double w[5] = {ctx->lap_c0, ctx->lap_c[0], ctx->lap_c[1], ctx->lap_c[2], ctx->lap_c[3]};
   return launch_stencil<double>(ctx, 1, x, ctx->n, prev, ctx->n, y, ctx->n, nullptr, w, nullptr, a, b, g,
-                                dot_partial, nblocks, st);
+                                dot_partial, nblocks, st, false, active);
 }
 
 // nonlocal.cu
