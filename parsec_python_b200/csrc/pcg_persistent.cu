@@ -37,8 +37,7 @@ __device__ __forceinline__ void grid_barrier(unsigned int* ctr, unsigned int tar
                                              long limit) {
   __syncthreads();
   if (threadIdx.x == 0) {
-    __threadfence();
-    atomicAdd(ctr, 1u);
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(ctr) : "memory");
     if (!failed) {
       long spins = 0;
       while (true) {
@@ -52,7 +51,6 @@ __device__ __forceinline__ void grid_barrier(unsigned int* ctr, unsigned int tar
         }
       }
     }
-    __threadfence();
   }
   __syncthreads();
 }
