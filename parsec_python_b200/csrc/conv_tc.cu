@@ -10,18 +10,25 @@
 // One CTA owns 128 output voxels (MMA M = 128) and all output channels (MMA
 // N = Cout rounded up to 16).  The reduction runs in stages of 64 entries:
 // one 128-byte row of BF16 per voxel, stored in the canonical K-major
-// 128-byte-swizzled layout, so one stage is four MMAs of K = 16.  The CTA's
-// threads gather stage s+1 into registers (16-byte pieces: 8 channels of one
-// tap) while the MMAs of stage s run; one thread issues the MMAs and commits
-// them to an mbarrier, the two-deep shared-memory ring reuses a buffer once
-// its MMAs have completed.  Warps 0-3 then read the accumulators back (TMEM
-// lane = voxel) and apply the bias and the activation.  Every wait is bounded
-// by the context's wait limit; on a timeout the CTA drains the MMAs it issued,
-// records status word 7 and writes nothing.
+// 128-byte-swizzled layout, so one stage is four MMAs of K = 16.  The gather
+// is bound by latency, not by bytes (a stage is 16 KB of L2 hits): the
+// threads copy 16-byte pieces (8 channels of one tap; zeros outside the grid)
+// asynchronously into a ring of CT_NS stages, CT_NS - 1 stages ahead of the
+// MMAs.  (With the one next stage held in registers the eight layers of a 90^3
+// pass took 742 us, with the ring 418.)  One thread
+// issues the MMAs of a stage and commits them to the stage's mbarrier; a
+// stage is refilled once its MMAs have completed.  The order of the MMAs, and
+// with it every bit of the result, does not depend on the ring.
+// Warps 0-3 then read the accumulators back (TMEM lane = voxel) and apply the
+// bias and the activation.  Every wait is bounded by the context's wait
+// limit; on a timeout the CTA drains the copies and MMAs it issued, records
+// status word 7 and writes nothing.
 #include "psc_internal.cuh"
 #include "../../include/psc.h"
 
 #include "conv_geom.cuh"
+
+#include <climits>
 
 namespace {
 constexpr int CT_NT = 256;                  // 8 warps gather; warps 0-3 also drain tensor memory
@@ -29,7 +36,7 @@ constexpr int CT_M = 128;                   // output voxels per CTA (MMA M)
 constexpr int CT_KS = 64;                   // reduction entries per stage (128 bytes of BF16)
 constexpr int CT_ATILE = CT_M * 128;        // 16 KB of gathered input per stage
 constexpr int CT_APER = CT_M * 8 / CT_NT;   // 16-byte input pieces per thread and stage
-constexpr int CT_BPER = 256 * 8 / CT_NT;    // 16-byte weight pieces per thread and stage (N <= 256)
+constexpr int CT_NS = 4;                    // stages of the shared-memory ring
 constexpr float CT_LEAK = 0.0625f;          // leaky-ReLU slope below zero (as the CUDA-core kernels)
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
@@ -74,6 +81,11 @@ __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity, long l
   return false;
 }
 
+// 16 bytes into shared memory, or zeros (src must be a valid address anyway)
+__device__ __forceinline__ void cp16(uint32_t dst, const void* src, bool in) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(in ? 16 : 0) : "memory");
+}
+
 __device__ __forceinline__ float conv_act(float a, int act) {
   return act == 1 ? fmaxf(a, 0.0f) : (act == 2 ? (a > 0.0f ? a : CT_LEAK * a) : a);
 }
@@ -91,12 +103,12 @@ __global__ void k_conv_wt(const __nv_bfloat16* __restrict__ W, int K, int Cout, 
 
 __global__ void __launch_bounds__(CT_NT, 1)
 k_conv_tc(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict__ S,
-          const __nv_bfloat16* __restrict__ Wt, const float* __restrict__ bias, ConvGeom g, int K, int Kpad, int N,
+          const __nv_bfloat16* __restrict__ Wt, const float* __restrict__ bias, ConvGeom g, int Kpad, int N,
           int act, __nv_bfloat16* __restrict__ out, float* __restrict__ out32, long wait_limit, int* status) {
   extern __shared__ unsigned char smraw[];
-  __shared__ __align__(8) uint64_t mbar[2];
+  __shared__ __align__(8) uint64_t mbar[CT_NS];
   __shared__ uint32_t s_tmem;
-  __shared__ int s_fail;
+  __shared__ int s_fail;   // stage at which the loop is left after a wait ran out (none: INT_MAX)
   unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smraw) + 1023) & ~uintptr_t(1023));
   const int warp = threadIdx.x >> 5;
   const int stage_bytes = CT_ATILE + N * 128;   // N is a multiple of 16: stages stay 1024-byte aligned
@@ -111,25 +123,39 @@ k_conv_tc(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict__
   const int c = threadIdx.x & 7;
   const int r0 = threadIdx.x >> 3;
   const int swz = (c ^ (r0 & 7)) << 4;   // the rows r0 + 32 u share r & 7
+  // Per row: the input voxel of tap (0, 0, 0), packed by axis, and which taps
+  // lie inside the grid (none for rows past the last voxel).  Everything that
+  // needs a division is done here once: with eight warps per SM a chain of
+  // integer divisions per stage took longer than the copies it addressed.
   int bx[CT_APER], by[CT_APER], bz[CT_APER];
-  bool vok[CT_APER];
+  uint32_t vmask[CT_APER];
 #pragma unroll
   for (int u = 0; u < CT_APER; ++u) {
     const long vo = vo0 + r0 + 32 * u;
-    vok[u] = vo < nvo;
-    const long v = vok[u] ? vo : 0;
+    const long v = vo < nvo ? vo : 0;
     const int xo = (int)(v % g.nxo);
     const long rr = v / g.nxo;
     const int yo = (int)(rr % g.nyo), zo = (int)(rr / g.nyo);
     bx[u] = xo * g.stride - pad;
     by[u] = yo * g.stride - pad;
     bz[u] = zo * g.stride - pad;
+    uint32_t m = 0;
+    for (int dz = 0; dz < ks; ++dz)
+      for (int dy = 0; dy < ks; ++dy)
+        for (int dx = 0; dx < ks; ++dx)
+          if ((unsigned)(bx[u] + dx) < (unsigned)g.nxi && (unsigned)(by[u] + dy) < (unsigned)g.nyi &&
+              (unsigned)(bz[u] + dz) < (unsigned)g.nzi)
+            m |= 1u << (dx + ks * (dy + ks * dz));
+    vmask[u] = vo < nvo ? m : 0u;
   }
+  // the next stage to gather: this thread's tap and first channel
+  int g_tap = (8 * c) / g.Cin, g_ci = 8 * c - g_tap * g.Cin;
+  int g_dx = g_tap % ks, g_dy = (g_tap / ks) % ks, g_dz = g_tap / (ks * ks);
+  const int ntap = ks * ks * ks;
 
   if (threadIdx.x == 0) {
-    s_fail = 0;
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&mbar[0])));
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&mbar[1])));
+    s_fail = INT_MAX;
+    for (int i = 0; i < CT_NS; ++i) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&mbar[i])));
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 0) {
@@ -142,77 +168,85 @@ k_conv_tc(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict__
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = s_tmem;
   const uint32_t idesc = idesc_bf16(N);
+  const uint32_t sbase = smem_u32(sm);
 
-  uint4 ra[CT_APER], rb[CT_BPER];
-  const uint4 zero4 = make_uint4(0u, 0u, 0u, 0u);
-  // the pieces of stage s: reduction entries kk .. kk+7 (one tap, 8 channels)
+  // copy the pieces of stage s (8 channels of one tap; stages in order) into
+  // its ring slot; one commit group per stage, empty past the end
   auto gather = [&](int s) {
-    const int kk = s * CT_KS + 8 * c;
-    const bool kin = kk < K;
-    const int tap = kin ? kk / g.Cin : 0;
-    const int ci = kk - tap * g.Cin;
-    const int dx = tap % ks, dy = (tap / ks) % ks, dz = tap / (ks * ks);
+    if (s < nstage) {
+      const uint32_t abuf = sbase + (uint32_t)((s % CT_NS) * stage_bytes);
+      const bool from_a = g_ci < g.Ca;
+      const int sh = from_a && g.up ? 1 : 0;
+      const int mx = from_a ? g.nxa : g.nxi, my = from_a ? g.nya : g.nyi;
+      const __nv_bfloat16* src = from_a ? A + g_ci : S + (g_ci - g.Ca);
+      const int ch = from_a ? g.Ca : g.Cs;
+      const uint32_t bit = g_tap < ntap ? 1u << g_tap : 0u;   // (past the last tap: padding, zeros)
 #pragma unroll
-    for (int u = 0; u < CT_APER; ++u) {
-      const int xi = bx[u] + dx, yi = by[u] + dy, zi = bz[u] + dz;
-      const bool in = kin && vok[u] && xi >= 0 && yi >= 0 && zi >= 0 && xi < g.nxi && yi < g.nyi && zi < g.nzi;
-      ra[u] = in ? conv_vin8(A, S, g, xi, yi, zi, ci) : zero4;
+      for (int u = 0; u < CT_APER; ++u) {
+        const bool in = (vmask[u] & bit) != 0u;
+        const long v = ((bx[u] + g_dx) >> sh) + (long)mx * (((by[u] + g_dy) >> sh) + my * ((bz[u] + g_dz) >> sh));
+        cp16(abuf + (uint32_t)((r0 + 32 * u) * 128 + swz), in ? src + v * ch : A, in);
+      }
+      const uint32_t bbuf = abuf + CT_ATILE;
+      const __nv_bfloat16* wsrc = Wt + s * CT_KS + 8 * c;
+      for (int row = r0; row < N; row += 32) cp16(bbuf + (uint32_t)(row * 128 + swz), wsrc + (long)row * Kpad, true);
+      for (g_ci += CT_KS; g_ci >= g.Cin; g_ci -= g.Cin) {
+        ++g_tap;
+        if (++g_dx == ks) {
+          g_dx = 0;
+          if (++g_dy == ks) {
+            g_dy = 0;
+            ++g_dz;
+          }
+        }
+      }
     }
-#pragma unroll
-    for (int u = 0; u < CT_BPER; ++u) {
-      const int row = r0 + 32 * u;
-      rb[u] = row < N ? __ldg(reinterpret_cast<const uint4*>(Wt + (long)row * Kpad + kk)) : zero4;
-    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
   };
 
   int last_commit = -1;   // thread 0: stage of the last MMA commit
-  if (nstage > 0) gather(0);
+  for (int s = 0; s < CT_NS - 1; ++s) gather(s);
   for (int s = 0; s < nstage; ++s) {
-    const int b = s & 1;
-    unsigned char* abuf = sm + b * stage_bytes;
-    unsigned char* bbuf = abuf + CT_ATILE;
-    if (s >= 2 && threadIdx.x == 0) {
-      // the MMAs of stage s-2 read this buffer: wait for their commit
-      if (!mbar_wait(smem_u32(&mbar[b]), (uint32_t)(((s - 2) >> 1) & 1), wait_limit)) s_fail = 1;
-    }
-    __syncthreads();
-    if (s_fail) break;
-#pragma unroll
-    for (int u = 0; u < CT_APER; ++u) *reinterpret_cast<uint4*>(abuf + (r0 + 32 * u) * 128 + swz) = ra[u];
-#pragma unroll
-    for (int u = 0; u < CT_BPER; ++u) {
-      const int row = r0 + 32 * u;
-      if (row < N) *reinterpret_cast<uint4*>(bbuf + row * 128 + swz) = rb[u];
-    }
-    if (s + 1 < nstage) gather(s + 1);
+    // this thread's pieces of stage s have landed; make them visible to the MMAs
+    asm volatile("cp.async.wait_group %0;" ::"n"(CT_NS - 2) : "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();
+    if (s >= s_fail) break;   // (set for this stage before its barrier: every thread leaves here)
     if (threadIdx.x == 0) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t aa = smem_u32(abuf), bb = smem_u32(bbuf);
+      const uint32_t aa = sbase + (uint32_t)((s % CT_NS) * stage_bytes), bb = aa + CT_ATILE;
 #pragma unroll
       for (int kk = 0; kk < CT_KS / 16; ++kk) {
         const uint32_t o = kk * 32;   // 16 BF16 = 32 bytes along K inside the swizzled row
         mma_bf16(tmem, sw128_desc(aa + o), sw128_desc(bb + o), idesc, (s > 0 || kk > 0) ? 1u : 0u);
       }
       asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                       smem_u32(&mbar[b]))
+                       smem_u32(&mbar[s % CT_NS]))
                    : "memory");
       last_commit = s;
     }
+    // stage s + CT_NS - 1 takes the slot of stage s - 1: its MMAs must be done
+    if (s >= 1 && s + CT_NS - 1 < nstage &&
+        !mbar_wait(smem_u32(&mbar[(s - 1) % CT_NS]), (uint32_t)(((s - 1) / CT_NS) & 1), wait_limit)) {
+      s_fail = s + 1;   // nothing is overwritten: every thread leaves after the next barrier
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    } else {
+      gather(s + CT_NS - 1);
+    }
   }
+  asm volatile("cp.async.wait_all;" ::: "memory");
   // the last commit covers every MMA issued before it; after a failed wait
   // the MMAs still in flight are drained before tensor memory is released
   if (threadIdx.x == 0 && last_commit >= 0) {
-    const uint32_t bar = smem_u32(&mbar[last_commit & 1]), par = (uint32_t)((last_commit >> 1) & 1);
-    if (s_fail || !mbar_wait(bar, par, wait_limit)) {
-      s_fail = 1;
+    const uint32_t bar = smem_u32(&mbar[last_commit % CT_NS]), par = (uint32_t)((last_commit / CT_NS) & 1);
+    if (s_fail != INT_MAX || !mbar_wait(bar, par, wait_limit)) {
+      s_fail = 0;
       mbar_wait(bar, par, PSC_DRAIN_WAIT);
     }
   }
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  if (s_fail) {
+  if (s_fail != INT_MAX) {
     if (threadIdx.x == 0) atomicExch(&status[7], 1);
   } else if (warp < 4) {
     // warp w owns tensor-memory lanes (= voxels) 32 w .. 32 w + 31
@@ -278,10 +312,10 @@ int psc_conv_tc_forward(psc_ctx* ctx, const ConvGeom& g, const __nv_bfloat16* a,
   auto* wt = static_cast<__nv_bfloat16*>(ctx->conv_wt);
   k_conv_wt<<<std::min(148 * 4, psc_div_up((long)N * Kpad, 256)), 256, 0, st>>>(w, K, g.Cout, N, Kpad, wt);
   PSC_LAUNCH_CHECK(ctx);
-  const size_t smem = 2 * (size_t)(CT_ATILE + N * 128) + 1024;
+  const size_t smem = CT_NS * (size_t)(CT_ATILE + N * 128) + 1024;   // at most 193 KB (N = 256)
   PSC_CUDA(ctx, cudaFuncSetAttribute(k_conv_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const long nvo = (long)g.nxo * g.nyo * g.nzo;
-  k_conv_tc<<<psc_div_up(nvo, CT_M), CT_NT, smem, st>>>(a, s, wt, bias, g, K, Kpad, N, act, o, out32,
+  k_conv_tc<<<psc_div_up(nvo, CT_M), CT_NT, smem, st>>>(a, s, wt, bias, g, Kpad, N, act, o, out32,
                                                        ctx->wait_limit, ctx->dev_status);
   PSC_LAUNCH_CHECK(ctx);
   return 0;

@@ -1,5 +1,6 @@
-// Learned initial density: BF16 3-D convolution kernels (forward, backward
-// data, backward weights) with FP32 accumulation, the loss and the Adam step.
+// Learned initial density: BF16 3-D convolution forward with FP32
+// accumulation on the CUDA cores, the C ABI of the convolutions (tensor-core
+// forward: conv_tc.cu, backward: conv_bwd.cu), the loss and the Adam step.
 //
 // The reference only consumes a predicted density (it reads a file in
 // V_ion/pseudoDiag_ML4Den_poisson.py:12-586 and renormalises it); the network
@@ -20,6 +21,8 @@
 #include <cuda_bf16.h>
 
 #include "conv_geom.cuh"
+
+#include <algorithm>
 
 namespace {
 
@@ -108,6 +111,148 @@ k_conv_fwd(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict_
     const float v = act == 1 ? fmaxf(a, 0.0f) : (act == 2 ? (a > 0.0f ? a : LEAK * a) : a);
     out[vo * g.Cout + co0 + j] = __float2bfloat16_rn(v);
     if (out32) out32[vo * g.Cout + co0 + j] = v;
+  }
+}
+
+// ---------------------------------------------------------------------------
+// forward of a stride-1 layer with 8 output channels per CTA (the full-grid
+// layers).  Four voxels of one x row (8 apart, so that a warp's loads are
+// consecutive) by 8 channels per thread: a weight fetched from shared memory
+// serves four voxels, the products are packed pairs of channels, and the
+// input brick with its halo is staged once for all the taps.  The plain
+// kernel above fetches two weight vectors per input value for eight
+// multiply-adds and reads the input 27 times through L1 (852 us for the three
+// layers of a 90^3 pass); this one takes 456 us and is bound by the FP32 pipe.  Every output adds its terms in k_conv_fwd<8>'s order (32
+// input channels at a time, taps, channels), so the results are the same
+// bits; a tap outside the grid adds a zero product instead of being skipped
+// (as in the tensor-core kernel).
+// ---------------------------------------------------------------------------
+constexpr int F8_X = 32, F8_Y = 4, F8_Z = 4;   // voxels per CTA (128 threads)
+
+// The taps of one staged chunk of NC channel octets.  Eight warps per SM do
+// not hide the shared-memory latency by themselves, so the weights of the next
+// input channel and the inputs of the next octet are loaded one step ahead of
+// the products (the weights lie in the order they are used in, and 8 floats
+// past the last ones belong to the CTA).
+template <int KS, int NC>
+__device__ __forceinline__ void fwd8_chunk(const uint4* x, int hx, int hxy, int hv, const float* wt,
+                                           float2 (&acc)[4][4]) {
+  float4 wa = *reinterpret_cast<const float4*>(wt), wb = *reinterpret_cast<const float4*>(wt + 4);
+  uint4 xv[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) xv[i] = x[8 * i];
+#pragma unroll 1
+  for (int r = 0; r < KS * KS; ++r) {
+    const uint4* xr = x + (r / KS) * hxy + (r % KS) * hx;
+    const int rn = r + 1 < KS * KS ? r + 1 : 0;
+    const uint4* xnext = x + (rn / KS) * hxy + (rn % KS) * hx;   // the row of taps after this one
+#pragma unroll
+    for (int dx = 0; dx < KS; ++dx)
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        const uint4* xp = c + 1 < NC ? xr + (c + 1) * hv + dx : (dx + 1 < KS ? xr + dx + 1 : xnext);
+        uint4 xn[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) xn[i] = xp[8 * i];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          wt += 8;
+          const float4 na = *reinterpret_cast<const float4*>(wt);
+          const float4 nb = *reinterpret_cast<const float4*>(wt + 4);
+          const float2 w2[4] = {make_float2(wa.x, wa.y), make_float2(wa.z, wa.w), make_float2(wb.x, wb.y),
+                                make_float2(wb.z, wb.w)};
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const uint32_t word = j / 2 == 0 ? xv[i].x : (j / 2 == 1 ? xv[i].y : (j / 2 == 2 ? xv[i].z : xv[i].w));
+            const float v = __uint_as_float(j & 1 ? word & 0xffff0000u : word << 16);
+#pragma unroll
+            for (int p = 0; p < 4; ++p) acc[i][p] = __ffma2_rn(make_float2(v, v), w2[p], acc[i][p]);
+          }
+          wa = na;
+          wb = nb;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) xv[i] = xn[i];
+      }
+  }
+}
+
+template <int KS>
+__global__ void __launch_bounds__(FWD_NT)
+k_conv_fwd8(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict__ S,
+            const __nv_bfloat16* __restrict__ W, const float* __restrict__ bias, ConvGeom g, int act, int nbx, int nby,
+            int aligned, __nv_bfloat16* __restrict__ out, float* __restrict__ out32) {
+  extern __shared__ __align__(16) unsigned char f8_sm[];
+  constexpr int PAD = KS / 2, TAPS = KS * KS * KS;
+  constexpr int HX = F8_X + 2 * PAD, HY = F8_Y + 2 * PAD, HZ = F8_Z + 2 * PAD, HV = HX * HY * HZ;
+  constexpr int CH = WTILE / 8;                        // input channels per chunk
+  const int nc_max = min(CH, g.Cin) / 8;
+  uint4* xs = reinterpret_cast<uint4*>(f8_sm);                      // [octet][HV]
+  float* ws = reinterpret_cast<float*>(xs + (size_t)nc_max * HV);   // [tap][channel of the chunk][8]
+  const int tx = threadIdx.x & 7, ty = (threadIdx.x >> 3) & 3, tz = threadIdx.x >> 5;
+  const int b = blockIdx.x;
+  const int x0 = (b % nbx) * F8_X, y0 = ((b / nbx) % nby) * F8_Y, z0 = (b / (nbx * nby)) * F8_Z;
+  const int co0 = blockIdx.y * 8;
+  float2 acc[4][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int p = 0; p < 4; ++p) acc[i][p] = make_float2(bias[co0 + 2 * p], bias[co0 + 2 * p + 1]);
+  const uint4 zero4 = make_uint4(0u, 0u, 0u, 0u);
+  for (int cc = 0; cc < g.Cin; cc += CH) {
+    const int cn = min(CH, g.Cin - cc), nc = cn / 8;
+    __syncthreads();
+    for (int e = threadIdx.x; e < nc * HV; e += FWD_NT) {
+      const int c = e / HV, w = e - c * HV;
+      const int x = x0 - PAD + w % HX, y = y0 - PAD + (w / HX) % HY, z = z0 - PAD + w / (HX * HY);
+      const bool in = x >= 0 && y >= 0 && z >= 0 && x < g.nxi && y < g.nyi && z < g.nzi;
+      xs[e] = in ? conv_vin8(A, S, g, x, y, z, cc + 8 * c) : zero4;
+    }
+    for (int e = threadIdx.x; e < TAPS * cn * 8; e += FWD_NT) {
+      const int co = e & 7, r = e >> 3, ci = r % cn, tap = r / cn;
+      ws[(tap * cn + ci) * 8 + co] = __bfloat162float(W[((long)tap * g.Cin + cc + ci) * g.Cout + co0 + co]);
+    }
+    __syncthreads();
+    const uint4* xt = xs + (tz * HY + ty) * HX + tx;
+    switch (nc) {
+      case 1: fwd8_chunk<KS, 1>(xt, HX, HX * HY, HV, ws, acc); break;
+      case 2: fwd8_chunk<KS, 2>(xt, HX, HX * HY, HV, ws, acc); break;
+      case 3: fwd8_chunk<KS, 3>(xt, HX, HX * HY, HV, ws, acc); break;
+      default: fwd8_chunk<KS, 4>(xt, HX, HX * HY, HV, ws, acc); break;
+    }
+  }
+  const int y = y0 + ty, z = z0 + tz;
+  if (y >= g.nyo || z >= g.nzo) return;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int x = x0 + tx + 8 * i;
+    if (x >= g.nxo) continue;
+    const long vo = x + (long)g.nxo * (y + (long)g.nyo * z);
+    float v[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float a = j & 1 ? acc[i][j >> 1].y : acc[i][j >> 1].x;
+      v[j] = act == 1 ? fmaxf(a, 0.0f) : (act == 2 ? (a > 0.0f ? a : LEAK * a) : a);
+    }
+    __nv_bfloat16* o = out + vo * g.Cout + co0;
+    if (aligned) {
+      uint4 pk;
+      __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&pk);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) h[j] = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
+      *reinterpret_cast<uint4*>(o) = pk;
+      if (out32) {
+        float4* q = reinterpret_cast<float4*>(out32 + vo * g.Cout + co0);
+        q[0] = make_float4(v[0], v[1], v[2], v[3]);
+        q[1] = make_float4(v[4], v[5], v[6], v[7]);
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        o[j] = __float2bfloat16_rn(v[j]);
+        if (out32) out32[vo * g.Cout + co0 + j] = v[j];
+      }
+    }
   }
 }
 
@@ -251,12 +396,26 @@ extern "C" int psc_conv3d_fwd(psc_ctx* ctx, const int* geom, const void* A, cons
   const auto* s = static_cast<const __nv_bfloat16*>(S);
   const auto* w = static_cast<const __nv_bfloat16*>(W);
   auto* o = static_cast<__nv_bfloat16*>(out);
-  // the tensor cores where a layer has 32 or more output channels; the
-  // full-grid layers with 8 (N padded to 16) are gather-bound and faster on
-  // the CUDA cores (90^3: 636 against 779 us for the widest of them)
+  // the tensor cores where a layer has 32 or more output channels; with 8 (N
+  // padded to 16) half of every MMA is padding and the gather costs as much as
+  // for 16, so the full-grid layers are faster on the CUDA cores (90^3: 40 -> 8
+  // channels 360 against 384 us, 8 -> 8 71 against 279).  Layers of stride 1 whose
+  // channels are no multiple of 16 take the eight-channel brick kernel, the
+  // rest (16 channels, stride 2) the plain one, whose 27 reads of a voxel hit L1.
   if (ctx->conv_tc == 2 || (ctx->conv_tc == 1 && g.Cout >= 32))
     return psc_conv_tc_forward(ctx, g, a, s, w, bias, act, o, out32, st);
-  if (g.Cout % 16 == 0) {
+  if (g.Cout % 16 != 0 && g.stride == 1) {
+    const int nbx = psc_div_up(g.nxo, F8_X), nby = psc_div_up(g.nyo, F8_Y), nbz = psc_div_up(g.nzo, F8_Z);
+    const int pad = g.ksize / 2, taps = g.ksize * g.ksize * g.ksize;
+    const size_t hv = (size_t)(F8_X + 2 * pad) * (F8_Y + 2 * pad) * (F8_Z + 2 * pad);
+    const int cn = std::min(WTILE / 8, g.Cin);
+    const int smem = (int)((size_t)(cn / 8) * hv * 16 + ((size_t)taps * cn + 1) * 8 * sizeof(float));
+    const int aligned = ((reinterpret_cast<uintptr_t>(o) | reinterpret_cast<uintptr_t>(out32)) & 15) == 0;
+    const dim3 grid(nbx * nby * nbz, g.Cout / 8);
+    auto kern = g.ksize == 3 ? k_conv_fwd8<3> : k_conv_fwd8<1>;
+    PSC_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    kern<<<grid, FWD_NT, smem, st>>>(a, s, w, bias, g, act, nbx, nby, aligned, o, out32);
+  } else if (g.Cout % 16 == 0) {
     dim3 grid(psc_div_up(nvo, FWD_NT), g.Cout / 16);
     k_conv_fwd<16><<<grid, FWD_NT, 0, st>>>(a, s, w, bias, g, act, o, out32);
   } else {
