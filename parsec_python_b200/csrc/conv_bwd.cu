@@ -34,10 +34,11 @@
 //                channels at a time.
 //
 // One training step's backward on 82^3 voxels (19 G multiply-adds for each
-// product): weights 8.3 -> 0.86 ms, inputs 3.6 -> 1.4 ms against one thread
+// product): weights 8.3 -> 0.76 ms, inputs 3.6 -> 0.92 ms against one thread
 // per weight (two shared-memory loads per multiply-add) and one thread per
-// voxel on the CUDA cores; the largest layer (192 -> 64 channels) runs its
-// weight gradient at 77 TFLOP/s of BF16 products.  What bounds them now is the
+// voxel on the CUDA cores.  (0.10 and 0.48 ms of
+// that were address arithmetic: a voxel's position is divided out once per
+// brick, not once per 16-byte piece.)  What bounds them now is the
 // mma.sync issue with its ldmatrix traffic (eight matrix loads per 24 MMAs)
 // and, on the coarse levels, too few bricks for 148 SMs.  Relative errors
 // against 64 bits over the network's layers: dW 7e-8 to 9e-8, input
@@ -242,19 +243,34 @@ k_conv_dw(DwArgs P) {
   for (int b = b0; b < b1; ++b) {
     const int bx = (b % P.nbx) * BX, by = ((b / P.nbx) % P.nby) * BY, bz = (b / (P.nbx * P.nby)) * BZ;
     __syncthreads();   // the previous brick is consumed
-    for (int e = threadIdx.x; e < nc8 * HV; e += CBW_NT) {
-      const int c = e / HV, w = e - c * HV;
-      const int x = bx * g.stride - pad + w % P.hx, y = by * g.stride - pad + (w / P.hx) % P.hy,
-                z = bz * g.stride - pad + w / (P.hx * P.hy);
-      Xs[e] = (x >= 0 && y >= 0 && z >= 0 && x < g.nxi && y < g.nyi && z < g.nzi)
-                  ? conv_vin8(P.A, P.S, g, x, y, z, 8 * (c8lo + c)) : zero4;
+    // a voxel's position is worked out once for all its channel octets
+    for (int w = threadIdx.x; w < HV; w += CBW_NT) {
+      const int wy = w / P.hx, wz = wy / P.hy;
+      const int x = bx * g.stride - pad + w - wy * P.hx, y = by * g.stride - pad + wy - wz * P.hy,
+                z = bz * g.stride - pad + wz;
+      const bool in = x >= 0 && y >= 0 && z >= 0 && x < g.nxi && y < g.nyi && z < g.nzi;
+      const long va = g.up ? (x >> 1) + (long)g.nxa * ((y >> 1) + (long)g.nya * (z >> 1))
+                           : x + (long)g.nxi * (y + (long)g.nyi * z);
+      const long vs = x + (long)g.nxi * (y + (long)g.nyi * z);
+      for (int c = 0; c < nc8; ++c) {
+        const int ch = 8 * (c8lo + c);
+        uint4 v = zero4;
+        if (in) v = *reinterpret_cast<const uint4*>(ch < g.Ca ? P.A + va * g.Ca + ch : P.S + vs * g.Cs + (ch - g.Ca));
+        Xs[c * HV + w] = v;
+      }
     }
-    for (int e = threadIdx.x; e < 3 * NT8 * BV; e += CBW_NT) {
-      const int j = e % NT8, v = (e / NT8) % BV, t = e / (NT8 * BV);
-      const int x = bx + v % BX, y = by + (v / BX) % BY, z = bz + v / (BX * BY);
-      const bool in = x < g.nxo && y < g.nyo && z < g.nzo && n0 / 8 + j < oct;
-      Gs[(t * NT8 + j) * BV + v] =
-          in ? P.planes[t * nvo * oct + (x + (long)g.nxo * (y + (long)g.nyo * z)) * oct + n0 / 8 + j] : zero4;
+    {
+      const int j = threadIdx.x % NT8;   // consecutive threads read a voxel's consecutive octets
+#pragma unroll
+      for (int q = 0; q < BV * NT8 / CBW_NT + (BV * NT8 < CBW_NT ? 1 : 0); ++q) {
+        const int v = threadIdx.x / NT8 + q * (CBW_NT / NT8);
+        if (v >= BV) break;
+        const int x = bx + v % BX, y = by + (v / BX) % BY, z = bz + v / (BX * BY);
+        const bool in = x < g.nxo && y < g.nyo && z < g.nzo && n0 / 8 + j < oct;
+        const uint4* src = P.planes + (x + (long)g.nxo * (y + (long)g.nyo * z)) * oct + n0 / 8 + j;
+#pragma unroll
+        for (int t = 0; t < 3; ++t) Gs[(t * NT8 + j) * BV + v] = in ? src[t * nvo * oct] : zero4;
+      }
     }
     __syncthreads();
 #pragma unroll 1
@@ -387,17 +403,31 @@ k_conv_dx(DxArgs P) {
 #pragma unroll
       for (int q = 0; q < 4; ++q) acc[i][j][q] = 0.0f;
 
+  // the brick voxels this thread stages (the same for every group of output
+  // channels): offsets into a plane, -1 outside the grid
+  const int lco = co8 - 1;   // log2 of co8 (1 or 2)
+  const int sc = threadIdx.x & lco, sw = threadIdx.x >> lco;
+  long goff[5];
+#pragma unroll
+  for (int q = 0; q < 5; ++q) {
+    const int w = sw + q * (CBW_NT >> lco);
+    const int x = cx - 1 + w % (DX + 2), y = cy - 1 + (w / (DX + 2)) % (DY + 2), z = cz - 1 + w / ((DX + 2) * (DY + 2));
+    const bool in = w < DH && x >= 0 && y >= 0 && z >= 0 && x < g.nxo && y < g.nyo && z < g.nzo;
+    goff[q] = in ? (x + (long)g.nxo * (y + (long)g.nyo * z)) * oct + sc : -1;
+  }
   for (int o0 = 0; o0 < oct; o0 += co8) {
     __syncthreads();
-    for (int e = threadIdx.x; e < 3 * co8 * DH; e += CBW_NT) {
-      const int c = e % co8, w = (e / co8) % DH, t = e / (co8 * DH);
-      const int x = cx - 1 + w % (DX + 2), y = cy - 1 + (w / (DX + 2)) % (DY + 2), z = cz - 1 + w / ((DX + 2) * (DY + 2));
-      const bool in = x >= 0 && y >= 0 && z >= 0 && x < g.nxo && y < g.nyo && z < g.nzo && o0 + c < oct;
-      Gs[(t * co8 + c) * DH + w] = in ? P.planes[t * nvo * oct + (x + (long)g.nxo * (y + (long)g.nyo * z)) * oct + o0 + c]
-                                      : zero4;
+#pragma unroll
+    for (int q = 0; q < 5; ++q) {
+      const int w = sw + q * (CBW_NT >> lco);
+      if (w >= DH) break;
+      const bool in = goff[q] >= 0 && o0 + sc < oct;
+#pragma unroll
+      for (int t = 0; t < 3; ++t)
+        Gs[(t * co8 + sc) * DH + w] = in ? P.planes[t * nvo * oct + goff[q] + o0] : zero4;
     }
     for (int e = threadIdx.x; e < 2 * usteps * NC; e += CBW_NT) {
-      const int c = e % co8, n = (e / co8) % NC, k = e / (co8 * NC);   // unit k co8 + c
+      const int c = e & lco, n = (e >> lco) % NC, k = (e >> lco) / NC;   // unit k co8 + c
       const int u = k * co8 + c;
       if (u >= 2 * usteps) continue;
       const bool in = u < units && ci0 + n < g.Cin && o0 + c < oct;
@@ -425,8 +455,8 @@ k_conv_dx(DxArgs P) {
         bf[NT8 - 1][1] = q[1];
       }
       const bool real = u < units;
-      const int c = real ? u % co8 : 0;
-      const int uo = real ? c * DH + s_off[u / co8] : 0;
+      const int c = real ? u & lco : 0;
+      const int uo = real ? c * DH + s_off[u >> lco] : 0;
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
         uint32_t a[3][4];
