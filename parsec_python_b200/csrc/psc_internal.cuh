@@ -184,7 +184,7 @@ struct psc_ctx {
   double* cg_x = nullptr;        // solution buffer the captured CG graph works on
   double* cg_p2 = nullptr;       // second direction buffer (the two alternate)
   double* cg_ro = nullptr;       // r.r before each iteration
-  unsigned int* cg_bar = nullptr;  // grid-barrier arrival counter of the persistent CG
+  unsigned int* cg_bar = nullptr;  // persistent CG: arrival counter, or the tagged sums of the box form
   int cg_persistent = 1;         // 1: persistent cooperative CG when the vectors fit in shared memory
   cudaGraphExec_t cg_exec = nullptr;
   cudaStream_t cap_stream = nullptr;  // private stream used only for graph capture
