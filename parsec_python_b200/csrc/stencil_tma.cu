@@ -6,18 +6,43 @@
 // column and a chunk of z planes.  For every plane the points it needs -- its
 // own S points plus R rows of y halo on each side -- are one contiguous range
 // of the plane, so a single cp.async.bulk (no tensor map, no multicast) moves
-// it into a slot of a ring of NBUF = R + 1 + D shared-memory windows (D = 3),
-// completing on the slot's mbarrier.  Each slot ends with one zero vector.
+// it into a slot of a ring of NBUF shared-memory windows, completing on the
+// slot's mbarrier.  Each slot ends with one zero vector.
 // The z neighbours of each point live in a register queue fed from the ring;
 // x and y neighbours are read from the current plane's window with 16-byte
 // loads (each thread owns a run of 2 FP64 or 4 FP32 points).  When the run
 // cannot cross a row edge (2 | nx for FP64, 4 | nx for FP32) the x vectors
 // outside the row are read from the zero vector, so the x terms need no
 // per-point masks; otherwise each point masks its x neighbours by its
-// distances to the row edges.  Prev and pot are prefetched three planes ahead
-// by per-thread 16-byte cp.async copies into a small shared-memory ring that
-// each thread reads back itself (no block-wide handshake).  D planes of X are
-// in flight per CTA at all times, which is what keeps HBM busy.
+// distances to the row edges.
+//
+// The kernel is bound by instruction issue before it is bound by HBM (the
+// FP32 step at 90^3, k = 307 moved 58 % of the copy rate at 62 % issue
+// active with 320 instructions per thread and plane, half of them moves,
+// selects and integer work), so everything around the 24 neighbour sums is
+// made to cost nothing inside the z loop:
+//   - the loop is unrolled by the queue length 2R + 1, so the queue rotates
+//     by renaming; ring offsets, barrier addresses and parities run along and
+//     wrap instead of being recomputed from the plane's number (opaque to the
+//     compiler, which otherwise keeps every sum of the unrolled pass in
+//     spilled registers);
+//   - whether Prev and the potential exist is a template argument, and the
+//     sphere mask of a point is an interval of planes found once;
+//   - x sums at odd distances are scalar adds: a packed add would first have
+//     to move both operands into aligned register pairs.
+// Prev and pot are copied three planes ahead by per-thread 16-byte cp.async
+// into a small ring that each thread reads back itself.  (Loading them, or
+// only the potential, two planes ahead into registers instead saves a few
+// instructions more and loses it all: 1.5 to 7.6 warps stalled on the loads
+// per issue.  Under full HBM load two planes are not early enough.)
+// With this a step at 90^3, k = 307 takes 635 us in FP32 and 1203 in FP64 (709
+// and 1346 before), and 34.5 instead of 40.6 us at 52^3, k = 27.  The limit now is the
+// shared-memory pipe, busy 77 % of the cycles: 24 neighbours of which the x and y
+// ones are loads.  (Giving a thread several rows, so that most y neighbours are
+// its own registers, cut the wavefronts by a fifth and was still slower: 1275 us
+// in FP64, with 12 warps per SM instead of 16 and twice the unrolled code.)
+// The order of the arithmetic of a point is fixed (shells from d = R down to
+// 1 for FP32), whatever the path.
 //
 // Every mbarrier wait is bounded by the context's wait limit: on timeout the
 // CTA records the failure in status[3], stops issuing copies and carries on
@@ -30,8 +55,7 @@
 #include <cmath>
 #include <cstdint>
 #include <cstring>
-#include <functional>
-#include <queue>
+#include <map>
 #include <type_traits>
 #include <vector>
 
@@ -44,25 +68,17 @@ constexpr int TNT = PSC_STENCIL_THREADS;  // threads per CTA
 #ifndef PSC_STENCIL_CTAS_PER_SM
 #define PSC_STENCIL_CTAS_PER_SM 2   // resident CTAs per SM (registers and shared memory)
 #endif
-// planes of X prefetched beyond the one consumed next
-#ifndef PSC_STENCIL_PREFETCH_F64
-#define PSC_STENCIL_PREFETCH_F64 3
-#endif
-#ifndef PSC_STENCIL_PREFETCH_F32
-#define PSC_STENCIL_PREFETCH_F32 3
-#endif
-#ifndef PSC_STENCIL_PP_SLOTS
-#define PSC_STENCIL_PP_SLOTS 4
-#endif
-template <typename T>
-__host__ __device__ constexpr int prefetch_depth() {
-  return sizeof(T) == 8 ? PSC_STENCIL_PREFETCH_F64 : PSC_STENCIL_PREFETCH_F32;
-}
-constexpr int PP_SLOTS = PSC_STENCIL_PP_SLOTS;  // Prev/pot slots: the plane in use + the prefetched
-#ifndef PSC_STENCIL_SYNC_EVERY
-#define PSC_STENCIL_SYNC_EVERY 2
-#endif
-constexpr int SYNC_EVERY = PSC_STENCIL_SYNC_EVERY;  // planes between block barriers
+// Planes between block barriers.  At 90^3, k = 307: 651 / 635 / 714 us per FP32
+// step for 2 / 3 / 4 (the ring runs dry), FP64 1203 / 1204 / 1303.
+constexpr int SYNC_EVERY = 3;
+// Planes of X in flight beyond the one consumed next (a template argument: the
+// ring's length as a variable cost 2.5 % in FP32): 3, the least that SYNC_EVERY
+// allows, or 5 for FP32 where that leaves room for two CTAs per SM (5 against 3
+// planes: 635 against 657 us at 90^3, 194 against 197 at 74^3; FP64 at 90^3 has
+// room for 3, and 2 cost 8 %).
+constexpr int AHEAD = SYNC_EVERY, AHEAD_F32 = 5;
+constexpr size_t SMEM_HALF = 113 * 1024;   // shared memory of one of two resident CTAs
+constexpr int PP_SLOTS = 4;   // Prev and pot: the plane in use + three in flight
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
@@ -221,26 +237,25 @@ struct TmaArgs {
 }  // namespace
 
 // YA: alignment (in elements) of the y-neighbour rows, the largest of VW, 2, 1
-// that divides nx; their loads are split to match.  MODE (FP32 only):
-// bit 0 = the arithmetic on packed pairs of points, bit 1 = sum-rule
-// correction: with the weights rounded to FP32 the sum rule c0 + 6 sum_d c_d
-// = 0 fails by their rounding errors (-6.1e-8 Ha at h = 0.47 bohr), a
-// constant shift of every eigenvalue that the band energy multiplies by the
-// electron count; one more term, -(that residual) x, removes it.  (Applying
-// every weight as its FP32 value plus its rounding error moved the
-// Rayleigh quotients of smooth fields by no more than this one term does.)
-template <typename T, int R, int YA, int VW, int MODE>
-__global__ void __launch_bounds__(TNT)
+// that divides nx; their loads are split to match.  PK (FP32): the arithmetic
+// on packed pairs of points.  HASP / HASV: Prev / the potential exist.
+// csr != 0 (FP32): sum-rule correction: with the weights rounded to FP32 the
+// sum rule c0 + 6 sum_d c_d = 0 fails by their rounding errors (-6.1e-8 Ha at
+// h = 0.47 bohr), a constant shift of every eigenvalue that the band energy
+// multiplies by the electron count; one more term, -(that residual) x,
+// removes it.  (Applying every weight as its FP32 value plus its rounding
+// error moved the Rayleigh quotients of smooth fields by no more than this one
+// term does.)
+template <typename T, int R, int YA, int VW, bool PK, bool HASP, bool HASV, int DEEP>
+__global__ void __launch_bounds__(TNT, PSC_STENCIL_CTAS_PER_SM)
 k_stencil_tma(TmaArgs<T> A) {
-  constexpr bool PK = (MODE & 1) != 0;
-  constexpr bool COMP = (MODE & 2) != 0;
   static_assert(!PK || (sizeof(T) == 4 && VW % 2 == 0), "packed pairs need FP32 runs of an even length");
-  static_assert(!COMP || sizeof(T) == 4, "compensated weights are for FP32");
   constexpr int TS = slab_points<VW>();    // points per slab (VW per thread)
-  constexpr int NBUF = R + 1 + prefetch_depth<T>();   // X plane windows resident
-  constexpr int NS = PP_SLOTS;
-  constexpr int Q = 2 * R + 1;             // z queue length
-  static_assert(SYNC_EVERY >= 1 && SYNC_EVERY <= NBUF - R, "barrier interval exceeds the ring");
+  constexpr int NBUF = R + 1 + DEEP;       // X plane windows resident
+  constexpr int Q = 2 * R + 1;             // z queue length, planes per unrolled pass
+  static_assert(SYNC_EVERY <= DEEP, "barrier interval exceeds the ring");
+  constexpr int NPP = (HASP ? 1 : 0) + (HASV ? 1 : 0);
+  static_assert((TS & (TS - 1)) == 0 && (PP_SLOTS & (PP_SLOTS - 1)) == 0, "the Prev/pot ring wraps by masking");
   constexpr int HV = (R + VW - 1) / VW;    // x-halo vectors on each side
   constexpr int NPV = 2 * HV + 1;          // x vectors per row (the centre one comes from the queue)
   constexpr int OFF = HV * VW;             // xs index of the thread's first point
@@ -253,9 +268,9 @@ k_stencil_tma(TmaArgs<T> A) {
   // that every slot starts where a bulk copy may write
   constexpr int Q16 = 16 / (int)sizeof(T);
   const int WS = (WIN + VW + Q16 - 1) / Q16 * Q16;
-  T* ring = reinterpret_cast<T*>(smem_raw);                                   // [NBUF][WS]
-  T* pring = ring + (size_t)NBUF * WS;                                        // [NS][2][TS]: Prev, pot
-  uint64_t* bars = reinterpret_cast<uint64_t*>(pring + (size_t)NS * 2 * TS);  // [NBUF]
+  T* ring = reinterpret_cast<T*>(smem_raw);                          // [NBUF][WS]
+  T* pring = ring + (size_t)NBUF * WS;                               // [PP_SLOTS][NPP][TS]: Prev, pot
+  uint64_t* bars = reinterpret_cast<uint64_t*>(pring + PP_SLOTS * NPP * TS);  // [NBUF]
   __shared__ int s_fail;
 
   const int4 work = A.sched[blockIdx.x];
@@ -278,9 +293,8 @@ k_stencil_tma(TmaArgs<T> A) {
   const int zlast = min(nz, z1 + R);  // X planes needed: [z0 - R, z1 + R) within [0, nz)
   const long col = work.x;
   const T* Xc = A.X + col * A.ldx;
-  const T* Pc = A.P ? A.P + col * A.ldp : nullptr;
+  const T* Pc = HASP ? A.P + col * A.ldp : nullptr;
   T* Yc = A.Y + col * A.ldy;
-  const bool has_pot = A.pot != nullptr;
 
   T ca, cb, cg;
   if (A.coef) { ca = (T)A.coef[0]; cb = (T)A.coef[1]; cg = (T)A.coef[2]; }
@@ -309,15 +323,14 @@ k_stencil_tma(TmaArgs<T> A) {
   }
   __syncthreads();
 
-  auto issue_x = [&](int p) {  // plane p into slot (p - z0) mod NBUF; only z0 <= p < zlast
-    const int s = (p - z0) % NBUF;
+  auto issue_x = [&](int p, int s) {  // plane p into slot s = (p - z0) mod NBUF; only z0 <= p < zlast
     uint64_t* bar = &bars[s];
     mbar_expect_tx(bar, xbytes);
     bulk_g2s(ring + (size_t)s * WS + (v0 - w0), Xc + (long)p * nxy + v0, xbytes, bar);
   };
   int issued = min(zlast, z0 + NBUF);  // next plane to copy (thread 0's count)
   if (threadIdx.x == 0) {
-    for (int p = z0; p < issued; ++p) issue_x(p);
+    for (int p = z0; p < issued; ++p) issue_x(p, p - z0);
   }
 
   // own run of VW points (it may cross a row boundary: every point has its own x)
@@ -326,23 +339,22 @@ k_stencil_tma(TmaArgs<T> A) {
   const int q = slab0 + loc;
   const int s_c = H + loc;  // window offset of the run
 
-  // Prev and pot of the run, NS-1 planes ahead: each thread copies its own
-  // 16-byte run with cp.async into slot (z - z0) mod NS and reads it back
-  // itself, so no block-wide handshake is needed.  One commit group per
-  // plane (empty ones too), so "wait until at most NS-2 groups are pending"
-  // means plane z has landed.  (P may alias Y: plane z of P is read before
-  // this thread stores plane z of Y.)
-  const bool use_pp = Pc || has_pot;
-  auto copy_pp = [&](int z) {
-    if (own && z < z1) {
-      T* d = pring + (size_t)((z - z0) % NS) * 2 * TS + loc;
-      if (Pc) cp_async_run<VW * sizeof(T)>(d, Pc + (long)z * nxy + q);
-      if (has_pot) cp_async_run<VW * sizeof(T)>(d + TS, A.pot + (long)z * nxy + q);
+  // Prev and pot of the run, PP_SLOTS - 1 planes ahead: each thread copies its
+  // own run into slot (z - z0) mod PP_SLOTS and reads it back itself, so no
+  // block-wide handshake is needed.  One commit group per plane (empty ones
+  // too), so "at most PP_SLOTS - 1 groups pending" means plane z has landed.
+  // (P may alias Y: plane z of P is read before this thread stores plane z of
+  // Y.)
+  constexpr int PSTEP = NPP * TS;
+  auto copy_pp = [&](bool in, int slot, int e) {   // element e of the column into the slot's elements
+    if (in) {
+      if constexpr (HASP) cp_async_run<VW * sizeof(T)>(pring + slot + loc, Pc + e);
+      if constexpr (HASV) cp_async_run<VW * sizeof(T)>(pring + slot + (HASP ? TS : 0) + loc, A.pot + e);
     }
     cp_async_commit();
   };
-  if (use_pp)
-    for (int z = z0; z < z0 + NS - 1; ++z) copy_pp(z);
+  if constexpr (NPP > 0)
+    for (int i = 0; i < PP_SLOTS - 1; ++i) copy_pp(own && z0 + i < z1, i * PSTEP, (z0 + i) * nxy + q);
 
   // z queue: planes below the chunk from global memory, z0 .. z0+R-1 from the ring
   T zq[VW][Q];
@@ -358,20 +370,25 @@ k_stencil_tma(TmaArgs<T> A) {
       for (int j = 0; j < VW; ++j) zq[j][i] = v[j];
     }
   }
-  bool fail = false;
-  int fail_plane = zlast;   // first plane whose wait this thread gave up on
+  // A limit of 0 polls gives up at once.  The first poll is the whole cost of
+  // a plane that has landed; the counted loop runs only when it has not.
+  bool fail = A.wait_limit <= 0;
+  int fail_plane = fail ? z0 : zlast;   // first plane whose wait this thread gave up on
+  auto wait_plane = [&](int p, uint64_t* bar, uint32_t parity) {
+    if (fail || mbar_try_wait(bar, parity)) return;
+    if (!mbar_wait(bar, parity, A.wait_limit)) {
+      fail = true;
+      fail_plane = p;
+    }
+  };
 #pragma unroll
   for (int i = 0; i < R; ++i) {
     const int p = z0 + i;
     if (p < nz) {
-      const int s = (p - z0) % NBUF;
-      if (!fail && !mbar_wait(&bars[s], ((p - z0) / NBUF) & 1, A.wait_limit)) {
-        fail = true;
-        fail_plane = p;
-      }
+      wait_plane(p, &bars[i], 0u);
       if (own) {
         T v[VW];
-        vload<VW>(ring + (size_t)s * WS + s_c, v);
+        vload<VW>(ring + (size_t)i * WS + s_c, v);
 #pragma unroll
         for (int j = 0; j < VW; ++j) zq[j][R + i] = v[j];
       }
@@ -418,17 +435,51 @@ k_stencil_tma(TmaArgs<T> A) {
       mB[p] = b_next ? (xp >= nx ? 1.f : 0.f) : mA[p];
     }
   }
+  // sphere mask: plane z of point j is inside iff zin[j] = lo | hi << 16 has
+  // lo <= z <= hi.  x^2 + y^2 + z^2 > r^2 is decided in FP64 as written; it
+  // grows with |z|, so the two ends are a square root and a step or two away.
   const bool masked = A.mask_r2 > 0.0;
-  double mxy[VW];   // (x^2 + y^2) of the run's points, for the sphere mask
+  uint32_t zin[VW];
 #pragma unroll
-  for (int j = 0; j < VW; ++j) {
-    const int qq = own ? q + j : 0;
-    const double xm = (qq % nx) * A.h - A.cx, ym = (qq / nx) * A.h - A.cy;
-    mxy[j] = xm * xm + ym * ym;
+  for (int j = 0; j < VW; ++j) zin[j] = 0u;
+  if (masked && own) {
+#pragma unroll 1
+    for (int j = 0; j < VW; ++j) {
+      const int qq = q + j;
+      const double xm = (qq % nx) * A.h - A.cx, ym = (qq / nx) * A.h - A.cy;
+      const double mxy = xm * xm + ym * ym;
+      auto inside = [&](int z) {
+        const double zm = z * A.h - A.cz;
+        return !(mxy + zm * zm > A.mask_r2);
+      };
+      const int zc = min(nz - 1, max(0, (int)(A.cz / A.h + 0.5)));   // the plane nearest the centre
+      int lo = 1, hi = 0;
+      if (inside(zc)) {
+        const int span = (int)fmin(sqrt(fmax(0.0, A.mask_r2 - mxy)) / A.h, (double)nz);
+        lo = max(0, zc - span);
+        while (lo > 0 && inside(lo - 1)) --lo;
+        while (lo < zc && !inside(lo)) ++lo;
+        hi = min(nz - 1, zc + span);
+        while (hi < nz - 1 && inside(hi + 1)) ++hi;
+        while (hi > zc && !inside(hi)) --hi;
+      }
+      const uint32_t v = (uint32_t)lo | ((uint32_t)hi << 16);
+#pragma unroll
+      for (int i = 0; i < VW; ++i)
+        if (i == j) zin[i] = v;
+    }
   }
   const T c0 = A.c0;
-  // z loop unrolled by Q so the register queue rotates by renaming:
-  // at unrolled position u, plane z - R + i lives in zq[.][(u + i) % Q]
+  const bool comp = sizeof(T) == 4 && A.csr != T(0);
+  // (a context's grid has fewer than 2^30 points)
+  int o = z0 * nxy + q;             // element of plane z
+  const int ring_end = NBUF * WS;
+  int ro = 0;                       // element of plane z's slot
+  int fo = R * WS;                  // of the queue front's slot (plane z + R; R < NBUF)
+  int fs = R;                       // that slot's number and parity
+  uint32_t fpar = 0;
+  int po = 0;                       // of plane z's Prev/pot slot
+  // at unrolled position u, plane z - R + i lies in zq[.][(u + i) % Q]
 #pragma unroll 1
   for (int zb = z0; zb < z1; zb += Q) {
 #pragma unroll
@@ -442,30 +493,22 @@ k_stencil_tma(TmaArgs<T> A) {
 #pragma unroll
         for (int j = 0; j < VW; ++j) f[j] = T(0);
         if (pf < nz) {
-          const int s = (pf - z0) % NBUF;
-          if (!fail && !mbar_wait(&bars[s], ((pf - z0) / NBUF) & 1, A.wait_limit)) {
-            fail = true;
-            fail_plane = pf;
-          }
-          if (own) vload<VW>(ring + (size_t)s * WS + s_c, f);
+          wait_plane(pf, bars + fs, fpar);
+          if (own) vload<VW>(ring + (fo + s_c), f);
         }
 #pragma unroll
         for (int j = 0; j < VW; ++j) zq[j][(u + 2 * R) % Q] = f[j];
       }
-      T pvv[VW], pov[VW];
-#pragma unroll
-      for (int j = 0; j < VW; ++j) pvv[j] = pov[j] = T(0);
-      if (use_pp) {
-        copy_pp(z + NS - 1);
-        cp_async_wait<NS - 1>();
-        if (own) {
-          const T* pp = pring + (size_t)((z - z0) % NS) * 2 * TS + loc;
-          if (Pc) vload<VW>(pp, pvv);
-          if (has_pot) vload<VW>(pp + TS, pov);
-        }
+      const T* pl = ring + ro;
+      T pv[VW], pt[VW];
+      if constexpr (NPP > 0) {
+        copy_pp(own && z + PP_SLOTS - 1 < z1, (po + (PP_SLOTS - 1) * PSTEP) & (PP_SLOTS * PSTEP - 1),
+                o + (PP_SLOTS - 1) * nxy);
+        cp_async_wait<PP_SLOTS - 1>();
       }
-      const T* pl = ring + (size_t)((z - z0) % NBUF) * WS;
       if (own) {
+        if constexpr (HASP) vload<VW>(pring + po + loc, pv);
+        if constexpr (HASV) vload<VW>(pring + po + (HASP ? TS : 0) + loc, pt);
         // x neighbours: the aligned vectors around the run (the run itself is
         // the queue's centre).  Row-aligned runs (EXACT) read the vectors
         // outside the row from the slot's zero pad; otherwise each point
@@ -482,17 +525,15 @@ k_stencil_tma(TmaArgs<T> A) {
         }
         auto xl = [&](int j, int d) -> T { return (EXACT || d <= el[j]) ? xs[OFF + j - d] : T(0); };
         auto xr = [&](int j, int d) -> T { return (EXACT || d <= er[j]) ? xs[OFF + j + d] : T(0); };
-        // per point: acc = c0 x + sum_d c_d (((y-d + y+d) + (z-d + z+d)) + (x-d + x+d)),
-        // and with compensated weights the same sum over the weights'
-        // rounding errors in its own (small) accumulator.  FP32 sums the
-        // shells from d = R down to 1 and adds c0 x last: of the orders
-        // tried this leaves the smallest bias in the Rayleigh quotients of
-        // smooth fields (the low spectrum), about 3e-9 Ha.
+        // per point: acc = c0 x + sum_d c_d (((y-d + y+d) + (z-d + z+d)) + (x-d + x+d)).
+        // FP32 sums the shells from d = R down to 1 and adds c0 x last: of
+        // the orders tried this leaves the smallest bias in the Rayleigh
+        // quotients of smooth fields (the low spectrum), about 3e-9 Ha.
         constexpr bool REV = sizeof(T) == 4;
-        T o[VW];
+        T out[VW];
         if constexpr (PK) {
-          constexpr int NP = VW / 2;
-          // the window masked for each owner pair (PAIRM): 16 multiplies
+          constexpr int NH = VW / 2;
+          // the window masked for each owner pair (PAIRM)
           float xa[PAIRM ? NPV * VW : 1], xb[PAIRM ? NPV * VW : 1];
           if constexpr (PAIRM) {
 #pragma unroll
@@ -502,9 +543,9 @@ k_stencil_tma(TmaArgs<T> A) {
               xb[i] = p == 3 ? xs[i] : xs[i] * mB[p];
             }
           }
-          float2 acc[NP];
+          float2 acc[NH];
 #pragma unroll
-          for (int h = 0; h < NP; ++h) {
+          for (int h = 0; h < NH; ++h) {
             const float2 xc = make_float2(xs[OFF + 2 * h], xs[OFF + 2 * h + 1]);
             acc[h] = REV ? make_float2(0.f, 0.f) : __fmul2_rn(make_float2(c0, c0), xc);
           }
@@ -517,34 +558,39 @@ k_stencil_tma(TmaArgs<T> A) {
             const float2 cd = make_float2(A.c[d - 1], A.c[d - 1]);
             const int sm = (u + R - d) % Q, sp = (u + R + d) % Q;
 #pragma unroll
-            for (int h = 0; h < NP; ++h) {
+            for (int h = 0; h < NH; ++h) {
               const int j = 2 * h;
               const float2 yy = __fadd2_rn(make_float2(ym[j], ym[j + 1]), make_float2(yp[j], yp[j + 1]));
               const float2 zz = __fadd2_rn(make_float2(zq[j][sm], zq[j + 1][sm]), make_float2(zq[j][sp], zq[j + 1][sp]));
               float2 xx;
               if constexpr (PAIRM) {
                 const float* xw = h == 0 ? xa : xb;
-                xx = __fadd2_rn(make_float2(xw[OFF + j - d], xw[OFF + j + 1 - d]),
-                                make_float2(xw[OFF + j + d], xw[OFF + j + 1 + d]));
-              } else {
+                if (d % 2 == 0)
+                  xx = __fadd2_rn(make_float2(xw[OFF + j - d], xw[OFF + j + 1 - d]),
+                                  make_float2(xw[OFF + j + d], xw[OFF + j + 1 + d]));
+                else
+                  xx = make_float2(xw[OFF + j - d] + xw[OFF + j + d], xw[OFF + j + 1 - d] + xw[OFF + j + 1 + d]);
+              } else if (EXACT && d % 2 == 0) {
                 xx = __fadd2_rn(make_float2(xl(j, d), xl(j + 1, d)), make_float2(xr(j, d), xr(j + 1, d)));
+              } else {
+                xx = make_float2(xl(j, d) + xr(j, d), xl(j + 1, d) + xr(j + 1, d));
               }
               const float2 t = __fadd2_rn(__fadd2_rn(yy, zz), xx);
               acc[h] = __ffma2_rn(cd, t, acc[h]);
             }
           }
 #pragma unroll
-          for (int h = 0; h < NP; ++h) {
+          for (int h = 0; h < NH; ++h) {
             const int j = 2 * h;
             const float2 xc = make_float2(xs[OFF + j], xs[OFF + j + 1]);
             float2 a = acc[h];
             if constexpr (REV) a = __ffma2_rn(make_float2(c0, c0), xc, a);
-            if constexpr (COMP) a = __ffma2_rn(make_float2(A.csr, A.csr), xc, a);
-            if (has_pot) a = __ffma2_rn(make_float2(pov[j], pov[j + 1]), xc, a);
+            if (comp) a = __ffma2_rn(make_float2(A.csr, A.csr), xc, a);
+            if constexpr (HASV) a = __ffma2_rn(make_float2(pt[j], pt[j + 1]), xc, a);
             float2 r = __ffma2_rn(make_float2(ca, ca), a, __fmul2_rn(make_float2(cb, cb), xc));
-            if (Pc) r = __ffma2_rn(make_float2(cg, cg), make_float2(pvv[j], pvv[j + 1]), r);
-            o[j] = r.x;
-            o[j + 1] = r.y;
+            if constexpr (HASP) r = __ffma2_rn(make_float2(cg, cg), make_float2(pv[j], pv[j + 1]), r);
+            out[j] = r.x;
+            out[j + 1] = r.y;
           }
         } else {
           T acc[VW];
@@ -569,27 +615,38 @@ k_stencil_tma(TmaArgs<T> A) {
             const T xc = xs[OFF + j];
             T a = acc[j];
             if constexpr (REV) a += c0 * xc;
-            if constexpr (COMP) a += A.csr * xc;
-            if (has_pot) a += pov[j] * xc;
-            o[j] = ca * a + cb * xc;
-            if (Pc) o[j] += cg * pvv[j];
+            if (comp) a += A.csr * xc;
+            if constexpr (HASV) a += pt[j] * xc;
+            out[j] = ca * a + cb * xc;
+            if constexpr (HASP) out[j] += cg * pv[j];
           }
         }
         if (masked) {
-          const double zm = z * A.h - A.cz;
 #pragma unroll
           for (int j = 0; j < VW; ++j)
-            if (mxy[j] + zm * zm > A.mask_r2) o[j] = T(0);
+            if (z < (int)(zin[j] & 0xffffu) || z > (int)(zin[j] >> 16)) out[j] = T(0);
         }
-        vstore<VW>(Yc + (long)z * nxy + q, o);
+        vstore<VW>(Yc + o, out);
       }
-      // every SYNC_EVERY planes (and after the last): the slots of all
-      // planes <= z are free, so the ring is topped up to plane z + NBUF.
-      // The queue front z + R stays covered while SYNC_EVERY <= NBUF - R.
-      if ((z - z0) % SYNC_EVERY == SYNC_EVERY - 1 || z == z1 - 1) {
+      o += nxy;
+      po = (po + PSTEP) & (PP_SLOTS * PSTEP - 1);
+      ro = ro + WS == ring_end ? 0 : ro + WS;
+      ++fs;
+      fo += WS;
+      if (fo == ring_end) {
+        fo = 0;
+        fs = 0;
+        fpar ^= 1u;
+      }
+      asm volatile("" : "+r"(ro), "+r"(fo), "+r"(po));
+      // every SYNC_EVERY planes, and at the end of the pass: the slots of the
+      // planes since the last barrier are free, so the ring is topped up to
+      // plane z + NBUF.  The queue front z + R stays covered while
+      // SYNC_EVERY <= NBUF - R.
+      if (u % SYNC_EVERY == SYNC_EVERY - 1 || u == Q - 1) {
         __syncthreads();
         if (threadIdx.x == 0 && !fail)
-          for (; issued < zlast && issued <= z + NBUF; ++issued) issue_x(issued);
+          for (; issued < zlast && issued <= z + NBUF; ++issued) issue_x(issued, (issued - z0) % NBUF);
       }
     }
   }
@@ -620,22 +677,35 @@ static bool tma_ok(const psc_ctx* ctx, const void* X, long ldx, const void* P, l
 // about in order as resident slots free up, so the table puts whole-column
 // (or half-column) items first and splits the last m (column, slab) pairs
 // into smaller z chunks that fill the final wave.  The split is the one with
-// the shortest simulated list-scheduling makespan over `slots` resident CTAs.
+// the shortest simulated list-scheduling makespan over `slots` resident CTAs
+// (every chunk of a split counted at its longest).
 static void z_chunks(int nz, int c, std::vector<int2>& out) {
   const int zc = (nz + c - 1) / c;
   out.clear();
   for (int z = 0; z < nz; z += zc) out.push_back(make_int2(z, std::min(nz, z + zc)));
 }
 
-static double makespan(const std::vector<int>& cost, int slots) {
-  std::priority_queue<double, std::vector<double>, std::greater<double>> q;
-  for (int i = 0; i < slots; ++i) q.push(0.0);
+// End of a greedy schedule of nb items of cost cb, then ns items of cost cs, on
+// `slots` equal workers.  Workers that are free at the same time form a level,
+// and all of a level take an item at once, so a schedule costs a few dozen
+// steps whatever the number of items (an item-by-item simulation of the
+// candidates took 27 ms at 307 columns, on every new grid context).
+static double makespan(long nb, double cb, long ns, double cs, int slots) {
+  std::map<double, long> level{{0.0, slots}};   // time -> workers free at it
   double end = 0.0;
-  for (int c : cost) {
-    const double t = q.top() + c;
-    q.pop();
-    q.push(t);
-    end = std::max(end, t);
+  for (int cls = 0; cls < 2; ++cls) {
+    long items = cls ? ns : nb;
+    const double c = cls ? cs : cb;
+    while (items > 0) {
+      const auto first = level.begin();
+      const double t = first->first;
+      const long take = std::min(items, first->second);
+      if (take == first->second) level.erase(first);
+      else first->second -= take;
+      level[t + c] += take;
+      end = std::max(end, t + c);
+      items -= take;
+    }
   }
   return end;
 }
@@ -647,7 +717,6 @@ static std::vector<int4> stencil_schedule(int nslab, int nz, int k, int fill, in
   int bb = 1, bs = 1;
   long bm = 0;
   std::vector<int2> cb, cs;
-  std::vector<int> cost;
   for (int b = 1; b <= std::min(2, cmax); ++b) {
     for (int sm = 1; sm <= 4; ++sm) {
       const int sc = std::min(cmax, b * sm);
@@ -657,12 +726,8 @@ static std::vector<int4> stencil_schedule(int nslab, int nz, int k, int fill, in
       const long step = std::max(1L, pairs / 32);
       for (long m = 0; m <= pairs; m += step) {
         if (sc == b && m > 0) break;
-        cost.clear();
-        for (long p = 0; p < pairs - m; ++p)
-          for (const int2& c : cb) cost.push_back(c.y - c.x + fill);
-        for (long p = 0; p < m; ++p)
-          for (const int2& c : cs) cost.push_back(c.y - c.x + fill);
-        const double t = makespan(cost, slots);
+        const double t = makespan((pairs - m) * (long)cb.size(), cb[0].y - cb[0].x + fill, m * (long)cs.size(),
+                                  cs[0].y - cs[0].x + fill, slots);
         if (t < best - 1e-9) {
           best = t;
           bb = b;
@@ -753,53 +818,83 @@ static const int4* stencil_sched(psc_ctx* ctx, int nslab, int k, int fill, int s
   return reinterpret_cast<const int4*>(b.dev);
 }
 
-template <typename T, int R, int VW, int MODE>
+template <typename T, int R, int YA, int VW, bool PK, bool HASP, bool HASV, int DEEP>
+static int launch_tma_k(psc_ctx* ctx, const TmaArgs<T>& A, int nwork, size_t smem, cudaStream_t st) {
+  auto kern = k_stencil_tma<T, R, YA, VW, PK, HASP, HASV, DEEP>;
+  PSC_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  kern<<<nwork, TNT, smem, st>>>(A);
+  PSC_LAUNCH_CHECK(ctx);
+  return 0;
+}
+
+template <typename T, int R, int VW, bool PK, int DEEP>
 static int launch_tma_t(psc_ctx* ctx, int k, const T* X, long ldx, const T* P, long ldp, T* Y, long ldy,
                         const T* pot, const double* w, const double* coef, double a, double b, double g,
-                        bool masked, cudaStream_t st) {
+                        bool masked, bool comp, cudaStream_t st) {
   const int nxy = ctx->nx * ctx->ny;
   constexpr int TS = slab_points<VW>();
   const int nslab = (nxy + TS - 1) / TS;
-  // each CTA pays a pipeline fill of about R + D planes; two CTAs per SM
+  constexpr size_t Q16 = 16 / sizeof(T);
+  const size_t win = (TS + 2 * (size_t)R * ctx->nx + VW + Q16 - 1) / Q16 * Q16;   // window + zero pad, 16-byte slots
+  const size_t npp = (P ? 1 : 0) + (pot ? 1 : 0);
+  const size_t slot = win * sizeof(T) + sizeof(uint64_t), pp = PP_SLOTS * npp * TS * sizeof(T);
+  const size_t smem = (R + 1 + DEEP) * slot + pp;
+  if (DEEP > AHEAD && smem > SMEM_HALF) return -1;   // (the caller comes back with AHEAD)
+  if (smem > 220 * 1024) return -1;  // window too wide: the register-queue kernel takes it
+  // each CTA pays a pipeline fill of about R + DEEP planes; two CTAs per SM
   // are resident (registers and shared memory)
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
   const int slots = PSC_STENCIL_CTAS_PER_SM * sms;
-  const int fill = R + prefetch_depth<T>() + 2;
+  const int fill = R + DEEP + 2;
   int nwork = 0;
   masked = masked && ctx->mask_r2 > 0.0;
   const int4* sched = stencil_sched(ctx, nslab, k, fill, slots, masked, TS, &nwork, st);
   PSC_REQUIRE(ctx, sched != nullptr, "stencil: work table allocation failed");
-  constexpr int NBUF = R + 1 + prefetch_depth<T>();
-  constexpr size_t Q16 = 16 / sizeof(T);
-  const size_t win = (TS + 2 * (size_t)R * ctx->nx + VW + Q16 - 1) / Q16 * Q16;   // window + zero pad, 16-byte slots
-  const size_t smem = (NBUF * win + (size_t)PP_SLOTS * 2 * TS) * sizeof(T) + NBUF * sizeof(uint64_t);
-  if (smem > 220 * 1024) return -1;  // window too wide: the register-queue kernel takes it
-  auto kern = (ctx->nx % VW == 0) ? k_stencil_tma<T, R, VW, VW, MODE>
-              : (ctx->nx % 2 == 0) ? k_stencil_tma<T, R, (VW >= 2 ? 2 : 1), VW, MODE>
-                                   : k_stencil_tma<T, R, 1, VW, MODE>;
-  PSC_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   TmaArgs<T> A;
   A.X = X; A.ldx = ldx; A.P = P; A.ldp = ldp; A.Y = Y; A.ldy = ldy; A.pot = pot;
   A.nx = ctx->nx; A.ny = ctx->ny; A.nz = ctx->nz; A.sched = sched;
   A.c0 = (T)w[0];
   // the sum rule c0 + 6 sum_d c_d = 0 holds for the FP64 weights; in the
   // stored type it is off by the weights' rounding errors, which the
-  // correction term removes (FP32 only, MODE bit 1)
+  // correction term removes (FP32 only)
   double rs = (double)A.c0 - w[0];
   for (int i = 0; i < 4; ++i) {
     A.c[i] = (T)w[1 + i];
     rs += 6.0 * ((double)A.c[i] - w[1 + i]);
   }
-  A.csr = (T)(-rs);
+  A.csr = comp ? (T)(-rs) : T(0);
   A.coef = coef; A.a = a; A.b = b; A.g = g; A.status = ctx->dev_status;
   A.wait_limit = ctx->wait_limit;
   A.mask_r2 = masked ? ctx->mask_r2 : 0.0;
   A.h = ctx->h;
   A.cx = ctx->mask_c[0]; A.cy = ctx->mask_c[1]; A.cz = ctx->mask_c[2];
-  kern<<<nwork, TNT, smem, st>>>(A);
-  PSC_LAUNCH_CHECK(ctx);
-  return 0;
+#define PSC_TMA_PV(YAV)                                                                         \
+  {                                                                                             \
+    if (P)                                                                                      \
+      return pot ? launch_tma_k<T, R, YAV, VW, PK, true, true, DEEP>(ctx, A, nwork, smem, st)         \
+                 : launch_tma_k<T, R, YAV, VW, PK, true, false, DEEP>(ctx, A, nwork, smem, st);       \
+    return pot ? launch_tma_k<T, R, YAV, VW, PK, false, true, DEEP>(ctx, A, nwork, smem, st)          \
+               : launch_tma_k<T, R, YAV, VW, PK, false, false, DEEP>(ctx, A, nwork, smem, st);        \
+  }
+  if constexpr (sizeof(T) == 4) {
+    // FP32 is the Hamiltonian's path alone, which always has a potential
+    PSC_REQUIRE(ctx, pot != nullptr, "stencil: FP32 blocks need the potential");
+#define PSC_TMA_P(YAV)                                                                       \
+  return P ? launch_tma_k<T, R, YAV, VW, PK, true, true, DEEP>(ctx, A, nwork, smem, st)            \
+           : launch_tma_k<T, R, YAV, VW, PK, false, true, DEEP>(ctx, A, nwork, smem, st);
+    if (ctx->nx % VW == 0) { PSC_TMA_P(VW) }
+    if constexpr (VW == 4) {   // (2-point runs are taken only where 2 divides nx)
+      if (ctx->nx % 2 == 0) { PSC_TMA_P(2) }
+      PSC_TMA_P(1)
+    }
+    return -1;
+#undef PSC_TMA_P
+  } else {
+    if (ctx->nx % VW == 0) PSC_TMA_PV(VW)
+    PSC_TMA_PV(1)
+  }
+#undef PSC_TMA_PV
 }
 
 // Returns -1 if the TMA path does not apply (caller uses the register kernel).
@@ -808,9 +903,10 @@ int psc_stencil_tma(psc_ctx* ctx, int k, const T* X, long ldx, const T* P, long 
                     const double* w, const double* coef, double a, double b, double g, bool masked,
                     cudaStream_t st) {
   if (!tma_ok<T>(ctx, X, ldx, P, ldp, Y, ldy)) return -1;
+  if (masked && ctx->nz > 0xffff) return -1;   // the mask's intervals are 16-bit planes
   // FP32 takes 4-point runs with the arithmetic on packed pairs (measured
   // fastest, also where nx is only 2-aligned and the x terms need per-point
-  // edge masks: 818 us per step at 90^3, k = 307, against 995-1055 us for
+  // edge masks: 818 us per step at 90^3, k = 307, when it was chosen, against 995-1055 us for
   // 2-point runs and 894 us for scalar arithmetic); impl 2 / 3 ask for
   // 2-point runs when nx is even but not a multiple of 4, impl 3 / 4 for
   // scalar arithmetic
@@ -820,24 +916,20 @@ int psc_stencil_tma(psc_ctx* ctx, int k, const T* X, long ldx, const T* P, long 
   // call's potential is not the FP32 potential that carries it
   const bool comp = ctx->stencil_comp == 1 ||
                     (ctx->stencil_comp == 2 && (const void*)pot != (const void*)ctx->pot32);
-  const int mode = (impl == 0 || impl == 2 ? 1 : 0) | (comp ? 2 : 0);
-#define PSC_TMA_ARGS ctx, k, X, ldx, P, ldp, Y, ldy, pot, w, coef, a, b, g, masked, st
-#define PSC_TMA_MODES(VWW)                                                                                    \
-  switch (mode) {                                                                                             \
-    case 0: return launch_tma_t<T, RR, VWW, 0>(PSC_TMA_ARGS);                                                 \
-    case 1: return launch_tma_t<T, RR, VWW, 1>(PSC_TMA_ARGS);                                                 \
-    case 2: return launch_tma_t<T, RR, VWW, 2>(PSC_TMA_ARGS);                                                 \
-    default: return launch_tma_t<T, RR, VWW, 3>(PSC_TMA_ARGS);                                                \
-  }
+  const bool pk = impl == 0 || impl == 2;
+#define PSC_TMA_ARGS ctx, k, X, ldx, P, ldp, Y, ldy, pot, w, coef, a, b, g, masked, comp, st
 #define PSC_TMA_R(RRV)                                                                                        \
   case RRV: {                                                                                                 \
     constexpr int RR = RRV;                                                                                   \
     if constexpr (sizeof(T) == 8)                                                                             \
-      return launch_tma_t<T, RR, 2, 0>(PSC_TMA_ARGS);                                                         \
-    else if (narrow) {                                                                                        \
-      PSC_TMA_MODES(2)                                                                                        \
-    } else {                                                                                                  \
-      PSC_TMA_MODES(4)                                                                                        \
+      return launch_tma_t<T, RR, 2, false, AHEAD>(PSC_TMA_ARGS);                                              \
+    else if (narrow)                                                                                          \
+      return pk ? launch_tma_t<T, RR, 2, true, AHEAD>(PSC_TMA_ARGS)                                           \
+                : launch_tma_t<T, RR, 2, false, AHEAD>(PSC_TMA_ARGS);                                         \
+    else {                                                                                                    \
+      if (!pk) return launch_tma_t<T, RR, 4, false, AHEAD>(PSC_TMA_ARGS);                                     \
+      const int rc = launch_tma_t<T, RR, 4, true, AHEAD_F32>(PSC_TMA_ARGS);                                   \
+      return rc >= 0 ? rc : launch_tma_t<T, RR, 4, true, AHEAD>(PSC_TMA_ARGS);                                \
     }                                                                                                         \
   }
   switch (ctx->radius) {
@@ -847,7 +939,6 @@ int psc_stencil_tma(psc_ctx* ctx, int k, const T* X, long ldx, const T* P, long 
     PSC_TMA_R(4)
   }
 #undef PSC_TMA_R
-#undef PSC_TMA_MODES
 #undef PSC_TMA_ARGS
   return -1;
 }
