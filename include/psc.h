@@ -108,8 +108,8 @@ int psc_apply_h_axpby(psc_ctx* ctx, int dtype, const void* X, long ldx, const vo
                       int k, double alpha, double beta, double gamma, void* stream);
 /* Stencil implementation: 0 = TMA-fed pipeline where the bulk-copy alignment
  * rules hold (default; 2-point FP64 runs, 4-point FP32 runs with the
- * arithmetic on packed pairs of points), 1 = register-queue kernel
- * everywhere, 2 = the TMA pipeline with 2-point FP32 runs when nx is even but
+ * arithmetic on packed pairs of points) and the bulk-copy kernel with shifted
+ * windows on the other grids, 1 = register-queue kernel everywhere, 2 = the TMA pipeline with 2-point FP32 runs when nx is even but
  * not a multiple of 4, 3 / 4 = as 2 / 0 with scalar FP32 arithmetic. */
 int psc_set_stencil_impl(psc_ctx* ctx, int impl);
 /* FP32 stencil weights.  Rounded to FP32 they break the sum rule

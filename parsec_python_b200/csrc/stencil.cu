@@ -171,6 +171,10 @@ int psc_stencil_tma(psc_ctx* ctx, int k, const T* X, long ldx, const T* P, long 
                     const double* w, const double* coef, double a, double b, double g, bool masked,
                     cudaStream_t st);
 
+template <typename T>
+int psc_stencil_bulk(psc_ctx* ctx, int k, const T* X, long ldx, const T* P, long ldp, T* Y, long ldy, const T* pot,
+                     const double* w, const double* coef, double a, double b, double g, cudaStream_t st);
+
 // Sphere mask: zero every point of k columns farther than sqrt(mask_r2)
 // from the cube's centre.
 template <typename T>
@@ -216,6 +220,13 @@ static int launch_stencil(psc_ctx* ctx, int k, const T* X, long ldx, const T* P,
                                      nblocks_out, st, false);
     if (rc) return rc;
     return psc_mask_block_impl(ctx, sizeof(T) == 8 ? PSC_F64 : PSC_F32, Y, ldy, k, st);
+  }
+  // grids whose planes the aligned pipeline cannot address: the bulk-copy
+  // kernel with shifted windows; the register-queue kernel has what is left
+  // (fused dot products, misaligned blocks, the widest windows, impl 1)
+  if (!dot_partial && ctx->stencil_impl != 1) {
+    const int rc = psc_stencil_bulk<T>(ctx, k, X, ldx, P, ldp, Y, ldy, pot, c0c, coef, a, b, g, st);
+    if (rc >= 0) return rc;
   }
   StencilPlan p = plan_stencil(ctx, k, sizeof(T));
   if (nblocks_out) *nblocks_out = (int)(p.grid.x * p.grid.y * p.grid.z);

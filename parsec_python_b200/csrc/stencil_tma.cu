@@ -818,6 +818,11 @@ static const int4* stencil_sched(psc_ctx* ctx, int nslab, int k, int fill, int s
   return reinterpret_cast<const int4*>(b.dev);
 }
 
+// the unmasked table for another kernel with the same (column, slab, z range) items
+const int4* psc_stencil_sched(psc_ctx* ctx, int nslab, int k, int fill, int slots, int* n, cudaStream_t st) {
+  return stencil_sched(ctx, nslab, k, fill, slots, false, 0, n, st);
+}
+
 template <typename T, int R, int YA, int VW, bool PK, bool HASP, bool HASV, int DEEP>
 static int launch_tma_k(psc_ctx* ctx, const TmaArgs<T>& A, int nwork, size_t smem, cudaStream_t st) {
   auto kern = k_stencil_tma<T, R, YA, VW, PK, HASP, HASV, DEEP>;
