@@ -265,18 +265,21 @@ __device__ __forceinline__ bool get_tagged(const unsigned long long* w, unsigned
 // spare the reductions that publish nothing the wait for their sum's store
 // before the arrival.  (Two forms without the counter lost: every CTA polling
 // every sum, and CTA 0 collecting them and handing the total back, 1.2 us more
-// per reduction.)  words: the counter, from word 16 on two per CTA.
+// per reduction.)  words: the counter, from word 16 on two per CTA for the odd
+// and two for the even reductions: a CTA may already store its next sum while
+// a slower one still reads this one, but not the one after.
 __device__ __forceinline__ double grid_reduce(double v, bool publish, unsigned long long* words, unsigned int tag,
                                               double* sh, double* bc, int* s_failed, long limit, int* status) {
   const int G = gridDim.x;
   asm volatile("" : "+l"(words));   // (opaque: nothing below is kept in registers between the calls)
   unsigned int* ctr = reinterpret_cast<unsigned int*>(words);
+  unsigned long long* sums = words + 16 + (tag & 1u ? 2 * G : 0);
   v = psc_block_sum<double, BOX_NT>(v, sh);
   if (threadIdx.x < 32) {
     bool ok = *s_failed == 0;   // (after a wait gave up there is no other)
     __syncwarp();
     if (threadIdx.x == 0) {
-      put_tagged(words + 16 + 2 * blockIdx.x, v, tag);
+      put_tagged(sums + 2 * blockIdx.x, v, tag);
       if (publish) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(ctr) : "memory");
       else asm volatile("red.relaxed.gpu.global.add.u32 [%0], 1;" ::"l"(ctr) : "memory");
       const unsigned int target = tag * (unsigned int)G;
@@ -297,12 +300,12 @@ __device__ __forceinline__ double grid_reduce(double v, bool publish, unsigned l
 #pragma unroll
       for (int q = 0; q < 5; ++q) {
         const int t = t0 + 32 * q + (int)threadIdx.x;
-        in[q] = t >= G || get_tagged(words + 16 + 2 * t, tag, &w[q]);
+        in[q] = t >= G || get_tagged(sums + 2 * t, tag, &w[q]);
       }
 #pragma unroll
       for (int q = 0; q < 5; ++q) {
         const int t = t0 + 32 * q + (int)threadIdx.x;
-        for (long i = 0; ok && !in[q] && i < limit; ++i) in[q] = get_tagged(words + 16 + 2 * t, tag, &w[q]);
+        for (long i = 0; ok && !in[q] && i < limit; ++i) in[q] = get_tagged(sums + 2 * t, tag, &w[q]);
         if (!in[q]) ok = false;
         if (t < G) s += w[q];
       }
@@ -489,7 +492,8 @@ k_cg_box(const double* __restrict__ rhs, double* __restrict__ xg, double* rg, in
 
 // The cut with the least work per iteration: about one cycle per point of the
 // largest box (two threads' slots of a warp per cycle, whole warps) and a
-// quarter per halo point; false if none fits shared memory, threads and runs.
+// quarter per halo point, and a run's own latency (of equal cuts the one with more
+// threads and shorter runs); false if none fits shared memory, threads and runs.
 static bool box_plan(const psc_ctx* ctx, int sms, size_t lim, BoxPlan* best, int* pt, size_t* smem) {
   const int R = ctx->radius, nx = ctx->nx, ny = ctx->ny, nz = ctx->nz;
   double cost = 1e300;
@@ -506,7 +510,7 @@ static bool box_plan(const psc_ctx* ctx, int sms, size_t lim, BoxPlan* best, int
       const long xn = (long)ncol * zs * zr;
       const size_t need = (slots + xn) * sizeof(double) + halo * (sizeof(int) + sizeof(unsigned short));
       if (slots > 65535 || need > lim) continue;
-      const double c = (double)((ncol * zs + 31) / 32 * 32) * zr + 0.25 * halo;
+      const double c = (double)((ncol * zs + 31) / 32 * 32) * zr + 0.25 * halo + 40.0 * zr;
       if (c < cost) {
         cost = c;
         *best = BoxPlan{px, py, pz, zs, (int)((halo + 1) / 2 * 2), (int)xn};
@@ -562,8 +566,8 @@ int psc_pcg_persistent(psc_ctx* ctx, const double* rhs, double* x, int maxit, do
   PSC_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem));
   if (per_sm < 1) return -1;
   if (!ctx->cg_r) PSC_CUDA(ctx, psc_dmalloc(&ctx->cg_r, n * sizeof(double)));
-  // the arrival counter, or the box kernel's words: 16 and 2 per CTA
-  const size_t bar_bytes = (16 + 2 * (size_t)sms) * sizeof(unsigned long long);
+  // the arrival counter, or the box kernel's words: 16 and 4 per CTA
+  const size_t bar_bytes = (16 + 4 * (size_t)sms) * sizeof(unsigned long long);
   if (!ctx->cg_bar) PSC_CUDA(ctx, psc_dmalloc(&ctx->cg_bar, bar_bytes));
   if (ctx->cg_part_cap < G) {
     psc_dfree(ctx->cg_part);

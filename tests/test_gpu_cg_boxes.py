@@ -37,3 +37,18 @@ def test_box_cg_matches_oracle(shape, order, maxit):
     assert its == its_o
     assert np.linalg.norm(x.cpu().numpy() - xo) <= 1e-9 * np.linalg.norm(xo)
     ctx.check_status()
+
+
+@pytest.mark.parametrize("n", [12, 40, 52])
+def test_repeated_solves_are_identical(n):
+    """Thousands of grid-wide reductions, in which fast CTAs run ahead of slow
+    ones: every solve ends, with the same bits."""
+    ctx = gpu.GridContext({"nx": n, "ny": n, "nz": n, "h": 0.34, "radius": 0.17 * (n - 1)}, 8)
+    g = torch.Generator(device="cuda").manual_seed(n)
+    rhs = torch.randn(ctx.n, dtype=torch.float64, device=DEV, generator=g)
+    x0, A = torch.zeros_like(rhs), gpu.Laplacian(ctx)
+    first, its = gpu.pcg(A, rhs, x0, 50, 1e-30)
+    for _ in range(150):
+        x, i = gpu.pcg(A, rhs, x0, 50, 1e-30)
+        assert i == its and torch.equal(x, first)
+    ctx.check_status()
