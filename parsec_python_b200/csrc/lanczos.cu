@@ -299,24 +299,19 @@ __device__ __forceinline__ void tri_lu(const double* __restrict__ a, const doubl
                                        double* __restrict__ du2, double* __restrict__ dl, double* __restrict__ piv) {
   double dc = a[0] - lam;
   double uc = k > 1 ? e[0] : 0.0;
+#pragma unroll 4
   for (int i = 0; i + 1 < k; ++i) {
     const double sub = e[i];
     const double dn = a[i + 1] - lam;
     const double un = i + 2 < k ? e[i + 1] : 0.0;
-    if (fabs(dc) >= fabs(sub)) {
-      const double d = fabs(dc) < tiny ? (dc < 0.0 ? -tiny : tiny) : dc;
-      const double r = 1.0 / d;
-      const double m = sub * r;
-      rd[i] = r; du[i] = uc; du2[i] = 0.0; dl[i] = m; piv[i] = 0.0;
-      dc = dn - m * uc;
-      uc = un;
-    } else {
-      const double r = 1.0 / sub;
-      const double m = dc * r;
-      rd[i] = r; du[i] = dn; du2[i] = un; dl[i] = m; piv[i] = 1.0;
-      dc = uc - m * dn;
-      uc = -m * un;
-    }
+    const bool swap = !(fabs(dc) >= fabs(sub));
+    const double d = fabs(dc) < tiny ? (dc < 0.0 ? -tiny : tiny) : dc;
+    const double r = 1.0 / (swap ? sub : d);
+    const double m = (swap ? dc : sub) * r;
+    rd[i] = r; du[i] = swap ? dn : uc; du2[i] = swap ? un : 0.0; dl[i] = m; piv[i] = swap ? 1.0 : 0.0;
+    const double up = swap ? uc : dn, low = swap ? dn : uc;
+    dc = up - m * low;
+    uc = swap ? -m * un : un;
   }
   const double d = fabs(dc) < tiny ? (dc < 0.0 ? -tiny : tiny) : dc;
   rd[k - 1] = 1.0 / d;
@@ -328,20 +323,19 @@ __device__ __forceinline__ void tri_lu_solve(double* __restrict__ x, int k, cons
                                              const double* __restrict__ dl, const double* __restrict__ piv) {
   // forward: apply the row interchanges and multipliers
   double xi = x[0];
-  for (int i = 0; i + 1 < k; ++i) {
-    const double xn = x[i + 1];
-    if (piv[i] == 0.0) {
-      x[i] = xi;
-      xi = xn - dl[i] * xi;
-    } else {
-      x[i] = xn;
-      xi = xi - dl[i] * xn;
-    }
+#pragma unroll 8
+  for (int i = 0; i + 1 < k; ++i) {   // (unrolled: the loads of later rows run ahead of the chain)
+    const double xn = x[i + 1], m = dl[i];
+    const bool swap = piv[i] != 0.0;
+    const double top = swap ? xn : xi, bot = swap ? xi : xn;
+    x[i] = top;
+    xi = bot - m * top;
   }
   x[k - 1] = xi;
   // backward with U (diagonal stored inverted)
   double x1 = x[k - 1] * rd[k - 1], x2 = 0.0;
   x[k - 1] = x1;
+#pragma unroll 8
   for (int i = k - 2; i >= 0; --i) {
     const double v = (x[i] - du[i] * x1 - du2[i] * x2) * rd[i];
     x[i] = v;
@@ -350,16 +344,138 @@ __device__ __forceinline__ void tri_lu_solve(double* __restrict__ x, int k, cons
   }
 }
 
-// Eigenvectors of the tridiagonal T by inverse iteration, one warp per
-// cluster of close eigenvalues (the members are orthogonalised against the
-// earlier ones).  With one warp per CTA (NT = 32) the LU factors and the
-// iterate live in shared memory (8k doubles with T); with NT = 128 the
-// factors go to `work` (5k doubles per cluster start) and the iterate to Z.
-template <int NT>
-__global__ void __launch_bounds__(NT)
-k_tri_invit(const double* __restrict__ ab, int k, const double* __restrict__ evals, int nvec, double* __restrict__ Z,
+// Eigenvectors of the tridiagonal T by inverse iteration: three solves each,
+// the members of a cluster of close eigenvalues orthogonalised against the
+// earlier ones after every solve.
+
+// the cluster [s0, s1) that eigenvalue j belongs to, and its shift: a member's
+// is at least pertol above the one before it
+__device__ __forceinline__ double tri_cluster(const double* __restrict__ evals, int nvec, int j, double ctol,
+                                              double pertol, int* s0, int* s1) {
+  int b = j, t = j + 1;
+  while (b > 0 && evals[b] - evals[b - 1] <= ctol) --b;
+  while (t < nvec && evals[t] - evals[t - 1] <= ctol) ++t;
+  double lam = evals[b];
+  for (int i = b + 1; i <= j; ++i) lam = fmax(evals[i], lam + pertol);
+  *s0 = b;
+  *s1 = t;
+  return lam;
+}
+
+// one warp: x to unit length, then x <- (T - lam I)^{-1} x
+__device__ __forceinline__ void tri_iterate(double* x, int k, int lane, const double* rd, const double* du,
+                                            const double* du2, const double* dl, const double* piv) {
+  const double nrm = sqrt(warp_dot_col(x, x, k, lane));
+  const double sc = nrm > 0.0 ? 1.0 / nrm : 1.0;
+  for (int i = lane; i < k; i += 32) x[i] *= sc;
+  __syncwarp();
+  if (lane == 0) tri_lu_solve(x, k, rd, du, du2, dl, piv);
+  __syncwarp();
+}
+
+// one warp: z = x at unit norm, its largest entry positive
+__device__ __forceinline__ void tri_finish(const double* x, double* z, int k, int lane) {
+  const double nrm = sqrt(warp_dot_col(x, x, k, lane));
+  double best = 0.0;
+  for (int i = lane; i < k; i += 32)
+    if (fabs(x[i]) > fabs(best)) best = x[i];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const double other = __shfl_xor_sync(0xffffffffu, best, o);
+    if (fabs(other) > fabs(best) || (fabs(other) == fabs(best) && other > best)) best = other;
+  }
+  const double sc = (best < 0.0 ? -1.0 : 1.0) / nrm;
+  for (int i = lane; i < k; i += 32) z[i] = x[i] * sc;
+  __syncwarp();
+}
+
+// one warp: x orthogonal to columns s0 .. j-1 of Z
+__device__ __forceinline__ void tri_orthogonalise(double* x, const double* Z, long ldz, int s0, int j, int k, int lane) {
+  for (int p = s0; p < j; ++p) {
+    const double* zp = Z + (long)p * ldz;
+    const double c = warp_dot_col(x, zp, k, lane);
+    for (int i = lane; i < k; i += 32) x[i] -= c * zp[i];
+    __syncwarp();
+  }
+}
+
+// Up to k = 512, two launches of one warp per eigenvalue with T, the factors
+// and the iterate in shared memory (8k doubles).  Everything that does not
+// need a cluster's earlier members is done for all eigenvalues at once: the
+// factors and the first solve (its result and the factors, 5k doubles, are left
+// in Z and `work`), or all three solves where the cluster is a single
+// eigenvalue.
+__global__ void __launch_bounds__(32)
+k_tri_invit_first(const double* __restrict__ ab, int k, const double* __restrict__ evals, int nvec,
+                  double* __restrict__ Z, long ldz, double crel, double* __restrict__ work) {
+  extern __shared__ double tri_sm[];
+  __shared__ double red[64];
+  __shared__ double s_lo, s_hi;
+  double* a = tri_sm;
+  double* e = tri_sm + k;
+  tri_load(ab, k, a, e, &s_lo, &s_hi, red);
+  const int lane = threadIdx.x, j = blockIdx.x;
+  // the floor keeps 1 / tiny and the squared iterates finite when T = 0
+  const double tnorm = fmax(fmax(fabs(s_lo), fabs(s_hi)), 1e-100);
+  int s0, s1;
+  const double lam = tri_cluster(evals, nvec, j, crel * tnorm, 10.0 * DBL_EPSILON * tnorm, &s0, &s1);
+  double* f = tri_sm + 2 * k;   // rd, du, du2, dl, piv
+  double* x = f + 5 * k;
+  if (lane == 0)
+    tri_lu(a, e, k, lam, fmax(DBL_EPSILON * tnorm, DBL_MIN), f, f + k, f + 2 * k, f + 3 * k, f + 4 * k);
+  for (int i = lane; i < k; i += 32) x[i] = tri_hash_unit(j, i);
+  __syncwarp();
+  double* z = Z + (long)j * ldz;
+  if (s1 - s0 == 1) {
+    for (int it = 0; it < 3; ++it) tri_iterate(x, k, lane, f, f + k, f + 2 * k, f + 3 * k, f + 4 * k);
+    tri_finish(x, z, k, lane);
+  } else {
+    tri_iterate(x, k, lane, f, f + k, f + 2 * k, f + 3 * k, f + 4 * k);
+    for (int i = lane; i < k; i += 32) z[i] = x[i];
+    double* w = work + (long)j * 5 * k;
+    for (int i = lane; i < 5 * k; i += 32) w[i] = f[i];
+  }
+}
+
+// The clusters of more than one eigenvalue, one warp each, from what
+// k_tri_invit_first left.  (One launch that took a cluster's factors and all its
+// solves in sequence, each step of a solve waiting for its own loads, took 1330
+// us at k = 307 and 103 at k = 55; the two take 721 and 71.)  A solve is a chain
+// of k dependent steps each way; a cluster's members still wait for each other.
+__global__ void __launch_bounds__(32)
+k_tri_invit_clusters(const double* __restrict__ ab, int k, const double* __restrict__ evals, int nvec, double* Z,
+                     long ldz, double crel, const double* __restrict__ work) {
+  extern __shared__ double tri_sm[];
+  __shared__ double red[64];
+  __shared__ double s_lo, s_hi;
+  tri_load(ab, k, tri_sm, tri_sm + k, &s_lo, &s_hi, red);
+  const int lane = threadIdx.x;
+  const double tnorm = fmax(fmax(fabs(s_lo), fabs(s_hi)), 1e-100);
+  int s0, s1;
+  tri_cluster(evals, nvec, blockIdx.x, crel * tnorm, 10.0 * DBL_EPSILON * tnorm, &s0, &s1);
+  if (s0 != (int)blockIdx.x || s1 - s0 == 1) return;
+  double* f = tri_sm;   // rd, du, du2, dl, piv (T is not needed any more)
+  double* x = f + 5 * k;
+  __syncwarp();
+  for (int j = s0; j < s1; ++j) {
+    double* z = Z + (long)j * ldz;
+    const double* w = work + (long)j * 5 * k;
+    for (int i = lane; i < 5 * k; i += 32) f[i] = w[i];
+    for (int i = lane; i < k; i += 32) x[i] = z[i];
+    __syncwarp();
+    for (int it = 0; it < 3; ++it) {
+      if (it > 0) tri_iterate(x, k, lane, f, f + k, f + 2 * k, f + 3 * k, f + 4 * k);
+      tri_orthogonalise(x, Z, ldz, s0, j, k, lane);
+    }
+    tri_finish(x, z, k, lane);
+  }
+}
+
+// Beyond: one launch, one warp per cluster, four to a CTA; the factors go to
+// `work` (5k doubles per cluster start) and the iterate to Z.
+__global__ void __launch_bounds__(128)
+k_tri_invit(const double* __restrict__ ab, int k, const double* __restrict__ evals, int nvec, double* Z,
             long ldz, double crel, double* __restrict__ work) {
-  constexpr bool SMEM = NT == 32;
   extern __shared__ double tri_sm[];
   __shared__ double red[64];
   __shared__ double s_lo, s_hi;
@@ -367,58 +483,27 @@ k_tri_invit(const double* __restrict__ ab, int k, const double* __restrict__ eva
   double* e = tri_sm + k;
   tri_load(ab, k, a, e, &s_lo, &s_hi, red);
   const int lane = threadIdx.x & 31;
-  const int s0 = blockIdx.x * (NT / 32) + (threadIdx.x >> 5);
-  if (s0 >= nvec) return;
-  // the floor keeps 1 / tiny and the squared iterates finite when T = 0
+  const int s = blockIdx.x * 4 + (threadIdx.x >> 5);
+  if (s >= nvec) return;
   const double tnorm = fmax(fmax(fabs(s_lo), fabs(s_hi)), 1e-100);
   const double ctol = crel * tnorm;
-  if (s0 > 0 && evals[s0] - evals[s0 - 1] <= ctol) return;  // not the first of its cluster
-  int s1 = s0 + 1;
-  while (s1 < nvec && evals[s1] - evals[s1 - 1] <= ctol) ++s1;
+  if (s > 0 && evals[s] - evals[s - 1] <= ctol) return;  // not the first of its cluster
+  int s0, s1;
+  double lam = tri_cluster(evals, nvec, s, ctol, 0.0, &s0, &s1);
   const double tiny = fmax(DBL_EPSILON * tnorm, DBL_MIN);
   const double pertol = 10.0 * DBL_EPSILON * tnorm;
-  double* rd = SMEM ? tri_sm + 2 * k : work + (long)s0 * 5 * k;
-  double* du = rd + k;
-  double* du2 = du + k;
-  double* dl = du2 + k;
-  double* piv = dl + k;
-  double lam_prev = 0.0;
+  double* f = work + (long)s0 * 5 * k;
   for (int j = s0; j < s1; ++j) {
-    double lam = evals[j];
-    if (j > s0) lam = fmax(lam, lam_prev + pertol);
-    lam_prev = lam;
-    double* z = Z + (long)j * ldz;
-    double* x = SMEM ? piv + k : z;
-    if (lane == 0) tri_lu(a, e, k, lam, tiny, rd, du, du2, dl, piv);
+    if (j > s0) lam = fmax(evals[j], lam + pertol);
+    double* x = Z + (long)j * ldz;
+    if (lane == 0) tri_lu(a, e, k, lam, tiny, f, f + k, f + 2 * k, f + 3 * k, f + 4 * k);
     for (int i = lane; i < k; i += 32) x[i] = tri_hash_unit(j, i);
     __syncwarp();
     for (int it = 0; it < 3; ++it) {
-      const double nrm = sqrt(warp_dot_col(x, x, k, lane));
-      const double sc = nrm > 0.0 ? 1.0 / nrm : 1.0;
-      for (int i = lane; i < k; i += 32) x[i] *= sc;
-      __syncwarp();
-      if (lane == 0) tri_lu_solve(x, k, rd, du, du2, dl, piv);
-      __syncwarp();
-      for (int p = s0; p < j; ++p) {
-        const double* zp = Z + (long)p * ldz;
-        const double c = warp_dot_col(x, zp, k, lane);
-        for (int i = lane; i < k; i += 32) x[i] -= c * zp[i];
-        __syncwarp();
-      }
+      tri_iterate(x, k, lane, f, f + k, f + 2 * k, f + 3 * k, f + 4 * k);
+      tri_orthogonalise(x, Z, ldz, s0, j, k, lane);
     }
-    // unit norm, largest entry positive
-    const double nrm = sqrt(warp_dot_col(x, x, k, lane));
-    double best = 0.0;
-    for (int i = lane; i < k; i += 32)
-      if (fabs(x[i]) > fabs(best)) best = x[i];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const double other = __shfl_xor_sync(0xffffffffu, best, o);
-      if (fabs(other) > fabs(best) || (fabs(other) == fabs(best) && other > best)) best = other;
-    }
-    const double sc = (best < 0.0 ? -1.0 : 1.0) / nrm;
-    for (int i = lane; i < k; i += 32) z[i] = x[i] * sc;
-    __syncwarp();
+    tri_finish(x, x, k, lane);
   }
 }
 
@@ -454,11 +539,14 @@ int psc_tridiag_eig_impl(psc_ctx* ctx, const double* ab, int k, int nvec, double
   }
   if (solo) {
     const size_t smem_iv = 8 * (size_t)k * sizeof(double);   // T, the LU factors and the iterate
-    if (tri_smem(ctx, (const void*)k_tri_invit<32>, smem_iv)) return 1;
-    k_tri_invit<32><<<nvec, 32, smem_iv, st>>>(ab, k, evals, nvec, Z, ldz, crel, ctx->tri_work);
+    if (tri_smem(ctx, (const void*)k_tri_invit_first, smem_iv)) return 1;
+    if (tri_smem(ctx, (const void*)k_tri_invit_clusters, smem_iv)) return 1;
+    k_tri_invit_first<<<nvec, 32, smem_iv, st>>>(ab, k, evals, nvec, Z, ldz, crel, ctx->tri_work);
+    PSC_LAUNCH_CHECK(ctx);
+    k_tri_invit_clusters<<<nvec, 32, smem_iv, st>>>(ab, k, evals, nvec, Z, ldz, crel, ctx->tri_work);
   } else {
-    if (tri_smem(ctx, (const void*)k_tri_invit<128>, smem)) return 1;
-    k_tri_invit<128><<<psc_div_up(nvec, 4), 128, smem, st>>>(ab, k, evals, nvec, Z, ldz, crel, ctx->tri_work);
+    if (tri_smem(ctx, (const void*)k_tri_invit, smem)) return 1;
+    k_tri_invit<<<psc_div_up(nvec, 4), 128, smem, st>>>(ab, k, evals, nvec, Z, ldz, crel, ctx->tri_work);
   }
   PSC_LAUNCH_CHECK(ctx);
   return 0;
