@@ -223,7 +223,7 @@ static int launch_stencil(psc_ctx* ctx, int k, const T* X, long ldx, const T* P,
   }
   // grids whose planes the aligned pipeline cannot address: the bulk-copy
   // kernel with shifted windows; the register-queue kernel has what is left
-  // (fused dot products, misaligned blocks, the widest windows, impl 1)
+  // (fused dot products, misaligned and small blocks, the widest windows, impl 1)
   if (!dot_partial && ctx->stencil_impl != 1) {
     const int rc = psc_stencil_bulk<T>(ctx, k, X, ldx, P, ldp, Y, ldy, pot, c0c, coef, a, b, g, st);
     if (rc >= 0) return rc;

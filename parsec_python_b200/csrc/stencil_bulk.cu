@@ -244,6 +244,13 @@ static int launch_bulk(psc_ctx* ctx, const BulkArgs<T>& A0, int k, cudaStream_t 
   BulkArgs<T> A = A0;
   const int S = BNT * PPT;
   const int nslab = (ctx->nx * ctx->ny + S - 1) / S;
+  // The register-queue kernel keeps the calls too small to fill this one's
+  // pipelines and the planes that leave a fifth of the slabs empty.  Measured
+  // (us, register / bulk): FP64 45 x 47 x 49 at 4 columns 11.8 / 14.8, at 8 18.9 /
+  // 16.9, at 64 142 / 84; 33 x 35 x 31 (slabs 75 % full) at 64 columns 36 / 47;
+  // FP32 61 x 55 x 67 at 4 columns 15.7 / 19.0, at 8 25.3 / 23.0; 45 x 47 x 49 (69 %
+  // full) at 64 columns 74 / 84.
+  if (ctx->n * k < (sizeof(T) == 8 ? 800000 : 1800000) || 5L * ctx->nx * ctx->ny < 4L * nslab * S) return -1;
   const size_t ws = ((size_t)S + 2 * (size_t)R * ctx->nx + 4 * G) / G * G;
   const size_t smem = (R + 4) * ws * sizeof(T) + (R + 4) * sizeof(uint64_t);
   if (smem > 110 * 1024) return -1;   // two CTAs per SM, or the register-queue kernel

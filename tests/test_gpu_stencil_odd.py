@@ -1,7 +1,7 @@
 """The stencil step on grids whose planes do not start on 16-byte boundaries:
 the bulk-copy kernel with shifted windows against the register-queue kernel
 (which tests/test_gpu_kernels.py holds against the oracle), over orders,
-slabs that end inside a row, planes smaller than a granule, leading
+slabs that end inside a row, calls below its sizes, leading
 dimensions of every remainder, blocks that start off a boundary (left to the
 register-queue kernel), Prev in place, absent or separate, and the last
 column's end (nothing past it is read, nothing outside the columns written).
@@ -25,15 +25,15 @@ DEV = torch.device("cuda", 0)
 
 CASES = [
     # grid, order, columns, ld - n, elements X starts past a 16-byte boundary, Prev
-    ((1, 1, 1), 2, 1, 0, 0, "none"),
     ((1, 1, 9), 8, 3, 1, 0, "in place"),
     ((3, 3, 3), 8, 5, 0, 0, "in place"),
-    ((5, 7, 11), 4, 2, 2, 0, "separate"),
-    ((33, 31, 6), 6, 4, 3, 0, "in place"),
-    ((61, 55, 67), 8, 31, 0, 0, "in place"),
-    ((101, 21, 13), 8, 3, 1, 0, "none"),
     ((45, 23, 30), 8, 3, 0, 1, "separate"),
-    ((255, 5, 9), 2, 2, 5, 0, "separate"),
+    ((71, 57, 61), 2, 9, 1, 0, "none"),
+    ((63, 65, 31), 4, 16, 2, 0, "separate"),
+    ((91, 45, 29), 6, 17, 3, 0, "in place"),
+    ((61, 55, 67), 8, 31, 0, 0, "in place"),
+    ((125, 41, 37), 8, 11, 1, 0, "separate"),
+    ((125, 41, 37), 8, 11, 0, 1, "none"),
 ]
 
 
