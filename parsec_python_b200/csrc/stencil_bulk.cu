@@ -15,7 +15,7 @@
 // cut to the boundary below it and the remaining elements are stored by one
 // thread before it arms the slot's barrier.
 //
-// H X at 61 x 55 x 67 with 31 columns: 124 -> 98 us, the step itself 101 -> 75.
+// H X at 61 x 55 x 67 with 31 columns: 124 -> 98 us, the step itself 101 -> 81.
 // Points of a thread are 256 apart, so shared-memory and global accesses of a
 // warp are consecutive without any alignment.  Waits are bounded as in
 // stencil_tma.cu (status word 3).
