@@ -6,7 +6,10 @@
  * index p = i + nx*(j + ny*k) (x fastest), zero Dirichlet values outside the
  * cube.  `stream` is a cudaStream_t passed as void*.  Every function returns
  * 0 on success, 2 for an invalid argument and 1 for a CUDA error; the message
- * is available from psc_last_error().  Units follow the reference: bohr,
+ * is available from psc_last_error().  The calls of one context share its
+ * scratch memory: calls that a program queues on different streams are
+ * ordered by it (an event, a synchronisation) unless each stream has a context
+ * of its own.  Units follow the reference: bohr,
  * Hartree for the Hamiltonian, Rydberg for XC potentials and energies.
  *
  * Each declaration names the part of PARSEC.py (zeyizhang-berkeley/

@@ -118,8 +118,8 @@ extern "C" int psc_ctx_create(int nx, int ny, int nz, double h, int fd_order, ps
   if ((e = psc_dmalloc(&ctx->red_partial, (size_t)PSC_RED_SLOTS * PSC_RED_BLOCKS * sizeof(double))) !=
       cudaSuccess)
     return fail(e, "partials");
-  if ((e = psc_dmalloc(&ctx->red_ticket, sizeof(unsigned int))) != cudaSuccess) return fail(e, "ticket");
-  if ((e = cudaMemset(ctx->red_ticket, 0, sizeof(unsigned int))) != cudaSuccess) return fail(e, "ticket");
+  if ((e = psc_dmalloc(&ctx->red_ticket, PSC_TICKETS * sizeof(unsigned int))) != cudaSuccess) return fail(e, "ticket");
+  if ((e = cudaMemset(ctx->red_ticket, 0, PSC_TICKETS * sizeof(unsigned int))) != cudaSuccess) return fail(e, "ticket");
   if ((e = psc_dmalloc(&ctx->scalars, 256 * sizeof(double))) != cudaSuccess) return fail(e, "scalars");
   if ((e = cudaMemset(ctx->scalars, 0, 256 * sizeof(double))) != cudaSuccess) return fail(e, "scalars");
   if ((e = pin_take(&ctx->host_scalars)) != cudaSuccess)
@@ -328,7 +328,7 @@ int psc_dots(psc_ctx* ctx, int nslots, const double* const* a, const double* con
   // one launch: the last CTA to finish sums the partials.  A CTA takes at
   // least 1024 entries, so short vectors do not pay for idle CTAs.
   const int nb = (int)std::max<long>(1, std::min<long>(PSC_RED_BLOCKS, (n + 1023) / 1024));
-  k_dots<256><<<nb, 256, 0, st>>>(args, nslots, n, ctx->red_partial, ctx->red_ticket, out_dev);
+  k_dots<256><<<nb, 256, 0, st>>>(args, nslots, n, ctx->red_partial, psc_ticket(ctx), out_dev);
   PSC_LAUNCH_CHECK(ctx);
   return 0;
 }

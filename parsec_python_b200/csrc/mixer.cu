@@ -217,7 +217,7 @@ extern "C" int psc_mixer_step(psc_ctx* ctx, const double* x1, const double* f1, 
   }
   double* dxl = ctx->mix_dx + (long)(m - 1) * n;
   double* dfl = ctx->mix_df + (long)(m - 1) * n;
-  k_mix_diff<<<nb, 256, 0, st>>>(x1, f1, dxl, dfl, ctx->mix_tmp, ctx->mix_ddf, n, ctx->mix_partial, ctx->red_ticket,
+  k_mix_diff<<<nb, 256, 0, st>>>(x1, f1, dxl, dfl, ctx->mix_tmp, ctx->mix_ddf, n, ctx->mix_partial, psc_ticket(ctx),
                                  fn + cur);
   PSC_LAUNCH_CHECK(ctx);
   const int mm = m - 1;
@@ -229,7 +229,7 @@ extern "C" int psc_mixer_step(psc_ctx* ctx, const double* x1, const double* f1, 
     PSC_CUDA(ctx, cudaEventRecord(ctx->mix_ev, st));
     const int nbd = (int)std::max<long>(1, std::min<long>(148, (n + MD_NT - 1) / MD_NT));
     k_mix_dots<<<nbd, MD_NT, 0, st>>>(ctx->mix_dx, ctx->mix_df, ctx->mix_ddf, f1, ctx->mix_tmp, n, mm,
-                                      ctx->mix_partial, ctx->red_ticket, ctx->mix_coef);
+                                      ctx->mix_partial, psc_ticket(ctx), ctx->mix_coef);
     PSC_LAUNCH_CHECK(ctx);
     PSC_CUDA(ctx, cudaEventSynchronize(ctx->mix_ev));
     const double fnorm = std::sqrt(ctx->host_scalars[120 + cur]);
@@ -245,7 +245,7 @@ extern "C" int psc_mixer_step(psc_ctx* ctx, const double* x1, const double* f1, 
   PSC_REQUIRE(ctx, m + 1 <= ctx->mix_cap, "mixer: history capacity exceeded (raise it at reset)");
   double* sv = ctx->mix_coef + 3 * ctx->mix_cap;
   k_mix_combine<<<nb, 256, 0, st>>>(ctx->mix_dx, ctx->mix_df, x1, f1, ctx->mix_tmp, ctx->mix_ddf, n, m, mix,
-                                    ctx->mix_coef, x_new, ctx->mix_nv, ctx->mix_partial, ctx->red_ticket, sv);
+                                    ctx->mix_coef, x_new, ctx->mix_nv, ctx->mix_partial, psc_ticket(ctx), sv);
   PSC_LAUNCH_CHECK(ctx);
   k_mix_final<<<nb, 256, 0, st>>>(ctx->mix_dx, ctx->mix_df, x1, f1, ctx->mix_nv, n, m, sv, x_new);
   PSC_LAUNCH_CHECK(ctx);

@@ -574,7 +574,7 @@ extern "C" int psc_pcg_poisson_prec(psc_ctx* ctx, const double* rhs, double* x, 
   if (rc) return rc;
   rc = spec_apply(ctx, r, p, nullptr, nullptr, nullptr, nullptr, nullptr, 0, zr, st);
   if (rc) return rc;
-  k_pcg_dir<<<1, PCG_NT, 0, st>>>(p, p, n, zr, ctx->nz, 1, maxit, tol, sc, ctx->red_ticket);
+  k_pcg_dir<<<1, PCG_NT, 0, st>>>(p, p, n, zr, ctx->nz, 1, maxit, tol, sc, psc_ticket(ctx));
   PSC_LAUNCH_CHECK(ctx);
   int queued = 0, its = 0;
   bool active = maxit > 0;
@@ -589,7 +589,7 @@ extern "C" int psc_pcg_poisson_prec(psc_ctx* ctx, const double* rhs, double* x, 
       if (rc) return rc;
       rc = spec_apply(ctx, r, z, sc, x, p, ap, ctx->cg_part, nblk, zr, st);
       if (rc) return rc;
-      k_pcg_dir<<<nb, PCG_NT, 0, st>>>(z, p, n, zr, ctx->nz, 0, maxit, tol, sc, ctx->red_ticket);
+      k_pcg_dir<<<nb, PCG_NT, 0, st>>>(z, p, n, zr, ctx->nz, 0, maxit, tol, sc, psc_ticket(ctx));
       PSC_LAUNCH_CHECK(ctx);
     }
     queued += batch;

@@ -10,6 +10,7 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <atomic>
 #include <cstdint>
 #include <cstdio>
 #include <string>
@@ -19,6 +20,7 @@
 #define PSC_MAX_K 1024        // widest subspace block accepted
 #define PSC_RED_BLOCKS 592    // fixed partial-sum count of the deterministic reductions (4 x 148 SMs)
 #define PSC_RED_SLOTS 16      // simultaneous dot products per reduction launch
+#define PSC_TICKETS 1024      // arrival counters of the reductions that end in their last CTA
 #define PSC_NORM_CHUNKS 32    // row chunks of the column-norm partial sums
 #define PSC_WAIT_DEFAULT (1L << 24)  // polls of a bounded device-side wait before it gives up
 #define PSC_DRAIN_WAIT (1L << 24)    // polls spent, after a failed wait, on copies and MMAs already issued
@@ -97,7 +99,8 @@ struct psc_ctx {
 
   // deterministic reductions
   double* red_partial = nullptr;  // [PSC_RED_SLOTS][PSC_RED_BLOCKS]
-  unsigned int* red_ticket = nullptr;  // arrival counter of the reductions that end in their last CTA
+  unsigned int* red_ticket = nullptr;  // [PSC_TICKETS] arrival counters, see psc_ticket
+  std::atomic<unsigned int> red_next{0};
   double* scalars = nullptr;      // general device scalar scratch [256]
   double* host_scalars = nullptr; // pinned host mirror [256]
 
@@ -306,7 +309,7 @@ __device__ __forceinline__ void psc_block_sums(double (&v)[NV], double* sh /* >=
 
 // True in every thread of the CTA that is last to get here: the partials that
 // the other CTAs' thread 0 wrote before are then visible (read them with
-// __ldcg).  The last CTA resets the ticket for the stream's next launch.
+// __ldcg).  The last CTA sets the counter back to zero.
 __device__ __forceinline__ bool psc_last_block(unsigned int* ticket) {
   __shared__ unsigned int s_last;
   if (threadIdx.x == 0) {
@@ -318,6 +321,14 @@ __device__ __forceinline__ bool psc_last_block(unsigned int* ticket) {
   }
   __syncthreads();
   return s_last != 0u;
+}
+
+// The arrival counter of one launch.  Every launch takes the next one of a
+// ring: were one word shared, launches that overlap on two streams would count
+// each other's CTAs, and a word left off zero would keep every later reduction
+// from ending.
+inline unsigned int* psc_ticket(psc_ctx* ctx) {
+  return ctx->red_ticket + ctx->red_next.fetch_add(1, std::memory_order_relaxed) % PSC_TICKETS;
 }
 
 // Sum of np partials by one warp: lane l adds part[l], part[l + 32], ... in

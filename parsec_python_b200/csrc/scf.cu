@@ -448,7 +448,7 @@ extern "C" int psc_lda_xc(psc_ctx* ctx, const double* rho, double* vxc, double h
   }
   PSC_REQUIRE(ctx, rho && vxc && out_dev, "psc_lda_xc: NULL pointer argument");
   cudaStream_t st = (cudaStream_t)stream;
-  k_xc<<<red_blocks(ctx->n), 256, 0, st>>>(rho, vxc, ctx->n, h3, ctx->red_partial, ctx->red_ticket, out_dev);
+  k_xc<<<red_blocks(ctx->n), 256, 0, st>>>(rho, vxc, ctx->n, h3, ctx->red_partial, psc_ticket(ctx), out_dev);
   PSC_LAUNCH_CHECK(ctx);
   return 0;
 }
@@ -494,7 +494,7 @@ extern "C" int psc_scf_update(psc_ctx* ctx, const double* ppot, const double* vx
   if (!ctx) return 2;
   cudaStream_t st = (cudaStream_t)stream;
   k_scf_update<<<red_blocks(ctx->n), 256, 0, st>>>(ppot, vxc, hpot, hpot0, rho, pot, pot_new, f, ctx->n,
-                                                  ctx->red_partial, ctx->red_ticket, out_dev);
+                                                  ctx->red_partial, psc_ticket(ctx), out_dev);
   PSC_LAUNCH_CHECK(ctx);
   return 0;
 }
