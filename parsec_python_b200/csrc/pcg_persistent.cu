@@ -265,15 +265,20 @@ __device__ __forceinline__ bool get_tagged(const unsigned long long* w, unsigned
 // spare the reductions that publish nothing the wait for their sum's store
 // before the arrival.  (Two forms without the counter lost: every CTA polling
 // every sum, and CTA 0 collecting them and handing the total back, 1.2 us more
-// per reduction.)  words: the counter, from word 16 on two per CTA for the odd
-// and two for the even reductions: a CTA may already store its next sum while
-// a slower one still reads this one, but not the one after.
+// per reduction.)
+//
+// A reduction that does not publish orders no memory access of other CTAs, so
+// nothing may rely on it alone to keep a write behind an earlier read: whatever
+// one CTA reads and another overwrites must have a publishing reduction in
+// between.  At least every second one publishes.  words: the counter, from
+// word 16 on two per CTA in each of four sets that take turns, so a sum is
+// overwritten four reductions later; r alternates between two arrays (k_cg_box).
 __device__ __forceinline__ double grid_reduce(double v, bool publish, unsigned long long* words, unsigned int tag,
                                               double* sh, double* bc, int* s_failed, long limit, int* status) {
   const int G = gridDim.x;
   asm volatile("" : "+l"(words));   // (opaque: nothing below is kept in registers between the calls)
   unsigned int* ctr = reinterpret_cast<unsigned int*>(words);
-  unsigned long long* sums = words + 16 + (tag & 1u ? 2 * G : 0);
+  unsigned long long* sums = words + 16 + (tag & 3u) * 2 * G;
   v = psc_block_sum<double, BOX_NT>(v, sh);
   if (threadIdx.x < 32) {
     bool ok = *s_failed == 0;   // (after a wait gave up there is no other)
@@ -328,8 +333,8 @@ __device__ __forceinline__ double grid_reduce(double v, bool publish, unsigned l
 
 template <int R, int PT>
 __global__ void __launch_bounds__(BOX_NT, 1)
-k_cg_box(const double* __restrict__ rhs, double* __restrict__ xg, double* rg, int nx, int ny, int nz, BoxPlan P,
-         double c0, double4 cw, unsigned long long* words, int* status, double tol, int maxit, double* out,
+k_cg_box(const double* __restrict__ rhs, double* __restrict__ xg, double* rg0, double* rg1, int nx, int ny, int nz,
+         BoxPlan P, double c0, double4 cw, unsigned long long* words, int* status, double tol, int maxit, double* out,
          long bar_limit) {
   extern __shared__ double sm[];
   __shared__ double sh[BOX_NT / 32];
@@ -436,7 +441,7 @@ k_cg_box(const double* __restrict__ rhs, double* __restrict__ xg, double* rg, in
   along_run([&](int i, double av, double) {
     const double ri = rhs[gb + i * nxy] - av;
     ap[i] = ri;   // (until every thread has read x)
-    rg[gb + i * nxy] = ri;
+    rg0[gb + i * nxy] = ri;
     rr += ri * ri;
   });
   __syncthreads();
@@ -453,7 +458,11 @@ k_cg_box(const double* __restrict__ rhs, double* __restrict__ xg, double* rg, in
     ++it;
     const bool alias = it <= 2;              // q = r in the first two iterations
     const double bt = it == 1 ? 0.0 : beta;  // p = r in the first
-    fill_halo(rg);
+    // r for the neighbours: read from one array, written to the other.  The
+    // one read here is written in the next iteration, behind this one's second
+    // reduction, which publishes.
+    const double* rin = it & 1 ? rg0 : rg1;
+    fill_halo(rin);
     __syncthreads();
     double pap = 0.0;
     along_run([&](int i, double sv, double rv) {
@@ -464,6 +473,7 @@ k_cg_box(const double* __restrict__ rhs, double* __restrict__ xg, double* rg, in
     pap = grid_reduce(pap, false, words, ++nred, sh, &bc[0], &s_failed, bar_limit, status);
     const double alp = ro / pap;
     rr = 0.0;
+    double* rout = it & 1 ? rg1 : rg0;
     int o = sb, g = gb, xo = tid;
     asm volatile("" : "+r"(o), "+r"(g), "+r"(xo));
 #pragma unroll
@@ -472,7 +482,7 @@ k_cg_box(const double* __restrict__ rhs, double* __restrict__ xg, double* rg, in
         xs[xo] += alp * p[i];
         const double ri = v[o] - alp * ap[i];
         v[o] = ri;
-        rg[g] = ri;
+        rout[g] = ri;
         rr += ri * ri;
       }
     const double ro1 = grid_reduce(rr, true, words, ++nred, sh, &bc[1], &s_failed, bar_limit, status);
@@ -566,8 +576,8 @@ int psc_pcg_persistent(psc_ctx* ctx, const double* rhs, double* x, int maxit, do
   PSC_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem));
   if (per_sm < 1) return -1;
   if (!ctx->cg_r) PSC_CUDA(ctx, psc_dmalloc(&ctx->cg_r, n * sizeof(double)));
-  // the arrival counter, or the box kernel's words: 16 and 4 per CTA
-  const size_t bar_bytes = (16 + 4 * (size_t)sms) * sizeof(unsigned long long);
+  // the arrival counter, or the box kernel's words: 16 and 8 per CTA
+  const size_t bar_bytes = (16 + 8 * (size_t)sms) * sizeof(unsigned long long);
   if (!ctx->cg_bar) PSC_CUDA(ctx, psc_dmalloc(&ctx->cg_bar, bar_bytes));
   if (ctx->cg_part_cap < G) {
     psc_dfree(ctx->cg_part);
@@ -579,6 +589,7 @@ int psc_pcg_persistent(psc_ctx* ctx, const double* rhs, double* x, int maxit, do
   const double4 cw = make_double4(ctx->lap_c[0], ctx->lap_c[1], ctx->lap_c[2], ctx->lap_c[3]);
   double* out = ctx->scalars + 80;
   double* rg = ctx->cg_r;
+  double* rg1 = ctx->cg_p;
   unsigned int* bar = ctx->cg_bar;
   auto* words = reinterpret_cast<unsigned long long*>(ctx->cg_bar);
   int* status = ctx->dev_status;
@@ -590,9 +601,9 @@ int psc_pcg_persistent(psc_ctx* ctx, const double* rhs, double* x, int maxit, do
   void* args[] = {(void*)&rhs, (void*)&x, (void*)&rg, (void*)&nx, (void*)&ny, (void*)&nz, (void*)&c0, (void*)&cw,
                   (void*)&chunk_i, (void*)&part, (void*)&bar, (void*)&status, (void*)&tol, (void*)&maxit, (void*)&out,
                   (void*)&bar_limit};
-  void* box_args[] = {(void*)&rhs, (void*)&x, (void*)&rg, (void*)&nx, (void*)&ny, (void*)&nz, (void*)&plan, (void*)&c0,
-                      (void*)&cw, (void*)&words, (void*)&status, (void*)&tol, (void*)&maxit, (void*)&out,
-                      (void*)&bar_limit};
+  void* box_args[] = {(void*)&rhs, (void*)&x, (void*)&rg, (void*)&rg1, (void*)&nx, (void*)&ny, (void*)&nz,
+                      (void*)&plan, (void*)&c0, (void*)&cw, (void*)&words, (void*)&status, (void*)&tol,
+                      (void*)&maxit, (void*)&out, (void*)&bar_limit};
   PSC_CUDA(ctx, cudaLaunchCooperativeKernel(fn, dim3(G), dim3(threads), box ? box_args : args, smem, st));
   PSC_LAUNCH_CHECK(ctx);
   PSC_CUDA(ctx, cudaMemcpyAsync(ctx->host_scalars + 80, out, 2 * sizeof(double), cudaMemcpyDeviceToHost, st));
