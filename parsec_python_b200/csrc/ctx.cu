@@ -24,36 +24,77 @@ extern "C" const char* psc_last_error(const psc_ctx* ctx) {
 
 // Pinned host scratch of the contexts (256 doubles each).  Pinning memory
 // takes a millisecond or more, as long as the rest of a context's creation, so
-// up to 16 blocks of destroyed contexts are kept for later ones.  A block has
-// no copy in flight when its context is destroyed: every entry point that
-// copies into it waits for the copy before it returns.
+// up to 16 blocks of destroyed contexts are kept for later ones, of the CUDA
+// context that pinned them only: cudaDeviceReset unpins and unmaps a device's
+// blocks, and what is pinned after it may lie at the same addresses.
+// A context that ended in an error may have a copy into its block in flight;
+// every call that succeeded has waited for its copies.
 constexpr size_t PIN_BYTES = 256 * sizeof(double);
-constexpr size_t PIN_KEEP = 16;
+constexpr int PIN_KEEP = 16;
+struct PinBlock {
+  double* p;
+  int device;
+  unsigned long long owner;   // id of the CUDA context that pinned it
+};
 static std::mutex g_pin_mu;
-// (never destroyed: a context may outlive the library's static objects)
-static std::vector<double*>& g_pin_free = *new std::vector<double*>;
+static PinBlock g_pin_free[PIN_KEEP];
+static int g_pin_count = 0;
 
-static cudaError_t pin_take(double** p) {
-  {
-    std::lock_guard<std::mutex> lk(g_pin_mu);
-    if (!g_pin_free.empty()) {
-      *p = g_pin_free.back();
-      g_pin_free.pop_back();
-      return cudaSuccess;
-    }
+// The current CUDA context's id, which no later context of the process
+// repeats (a reset makes a new one); 0 if the driver does not tell.
+static unsigned long long cuda_context_id() {
+  using GetId = int (*)(void* context, unsigned long long* id);   // cuCtxGetId
+  void* fn = nullptr;
+  cudaDriverEntryPointQueryResult found;
+  unsigned long long id = 0;
+  if (cudaGetDriverEntryPoint("cuCtxGetId", &fn, cudaEnableDefault, &found) != cudaSuccess ||
+      found != cudaDriverEntryPointSuccess || !fn || reinterpret_cast<GetId>(fn)(nullptr, &id) != 0) {
+    cudaGetLastError();
+    return 0;
   }
-  return cudaHostAlloc(reinterpret_cast<void**>(p), PIN_BYTES, cudaHostAllocPortable);
+  return id;
 }
 
-static void pin_give(double* p) {
-  if (!p) return;
+static cudaError_t pin_take(psc_ctx* ctx) {
+  ctx->host_owner = cuda_context_id();
+  ctx->host_scalars = nullptr;
   {
     std::lock_guard<std::mutex> lk(g_pin_mu);
-    if (g_pin_free.size() < PIN_KEEP) {
-      g_pin_free.push_back(p);
+    for (int i = g_pin_count; i-- > 0;) {
+      const PinBlock b = g_pin_free[i];
+      if (b.device != ctx->device) continue;
+      g_pin_free[i] = g_pin_free[--g_pin_count];
+      if (b.owner == ctx->host_owner) {
+        ctx->host_scalars = b.p;
+        break;
+      }
+      // (of a context that a reset has ended: the memory went with it)
+    }
+  }
+  if (!ctx->host_scalars) {
+    const cudaError_t e =
+        cudaHostAlloc(reinterpret_cast<void**>(&ctx->host_scalars), PIN_BYTES, cudaHostAllocPortable);
+    if (e != cudaSuccess) return e;
+  }
+  std::memset(ctx->host_scalars, 0, PIN_BYTES);
+  return cudaSuccess;
+}
+
+static void pin_give(psc_ctx* ctx) {
+  double* p = ctx->host_scalars;
+  ctx->host_scalars = nullptr;
+  if (!p) return;
+  if (ctx->host_owner != 0 && ctx->last_error.empty()) {
+    std::lock_guard<std::mutex> lk(g_pin_mu);
+    if (g_pin_count < PIN_KEEP) {
+      g_pin_free[g_pin_count++] = PinBlock{p, ctx->device, ctx->host_owner};
       return;
     }
   }
+  int dev = -1;
+  if (ctx->host_owner != 0 && cudaGetDevice(&dev) == cudaSuccess && dev == ctx->device &&
+      cuda_context_id() != ctx->host_owner)
+    return;   // a reset has unpinned it
   cudaFreeHost(p);
 }
 
@@ -122,7 +163,7 @@ extern "C" int psc_ctx_create(int nx, int ny, int nz, double h, int fd_order, ps
   if ((e = cudaMemset(ctx->red_ticket, 0, PSC_TICKETS * sizeof(unsigned int))) != cudaSuccess) return fail(e, "ticket");
   if ((e = psc_dmalloc(&ctx->scalars, 256 * sizeof(double))) != cudaSuccess) return fail(e, "scalars");
   if ((e = cudaMemset(ctx->scalars, 0, 256 * sizeof(double))) != cudaSuccess) return fail(e, "scalars");
-  if ((e = pin_take(&ctx->host_scalars)) != cudaSuccess)
+  if ((e = pin_take(ctx)) != cudaSuccess)
     return fail(e, "host scalars");
   if ((e = psc_dmalloc(&ctx->dev_status, 8 * sizeof(int))) != cudaSuccess) return fail(e, "status");
   if ((e = cudaMemset(ctx->dev_status, 0, 8 * sizeof(int))) != cudaSuccess) return fail(e, "status");
@@ -148,7 +189,7 @@ extern "C" int psc_ctx_destroy(psc_ctx* ctx) {
   for (auto& s : ctx->species) free_species(s);
   psc_free_projectors(ctx);
   psc_dfree(ctx->pot64); psc_dfree(ctx->pot32); psc_dfree(ctx->cheb_coef); psc_dfree(ctx->red_partial);
-  psc_dfree(ctx->red_ticket); psc_dfree(ctx->scalars); pin_give(ctx->host_scalars); psc_dfree(ctx->dev_status);
+  psc_dfree(ctx->red_ticket); psc_dfree(ctx->scalars); pin_give(ctx); psc_dfree(ctx->dev_status);
   psc_dfree(ctx->gram); psc_dfree(ctx->gram2); psc_dfree(ctx->evec); psc_dfree(ctx->tri);
   psc_dfree(ctx->gram_partial); psc_dfree(ctx->lz_v); psc_dfree(ctx->cg_r); psc_dfree(ctx->cg_p);
   psc_dfree(ctx->cg_ap); psc_dfree(ctx->cg_part); psc_dfree(ctx->mix_dx); psc_dfree(ctx->mix_df);

@@ -103,6 +103,7 @@ struct psc_ctx {
   std::atomic<unsigned int> red_next{0};
   double* scalars = nullptr;      // general device scalar scratch [256]
   double* host_scalars = nullptr; // pinned host mirror [256]
+  unsigned long long host_owner = 0;   // id of the CUDA context that pinned it (0 unknown)
 
   // small dense work (k x k)
   int dense_cap = 0;
