@@ -315,7 +315,7 @@ extern "C" int psc_pcg_poisson(psc_ctx* ctx, const double* rhs, double* x, int m
     if (ctx->host_scalars[CG_ACTIVE] == 0.0) break;
   }
   PSC_CUDA(ctx, cudaMemcpyAsync(x, ctx->cg_x, n * sizeof(double), cudaMemcpyDeviceToDevice, st));
-  if (its_out) *its_out = (int)ctx->host_scalars[CG_ITS];
+  if (its_out) *its_out = maxit > 0 ? (int)ctx->host_scalars[CG_ITS] : 0;   // (no state was read for none)
   return 0;
 }
 
