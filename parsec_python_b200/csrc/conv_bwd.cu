@@ -529,7 +529,7 @@ k_sum_chunks(const float* __restrict__ part, int nchunk, long nw, float* __restr
 
 template <int NT8, int MT>
 static int launch_dw(psc_ctx* ctx, const DwArgs& P, dim3 grid, size_t smem, cudaStream_t st) {
-  PSC_CUDA(ctx, cudaFuncSetAttribute(k_conv_dw<NT8, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  PSC_CUDA(ctx, psc_smem_optin(k_conv_dw<NT8, MT>));
   k_conv_dw<NT8, MT><<<grid, CBW_NT, smem, st>>>(P);
   PSC_LAUNCH_CHECK(ctx);
   return 0;
@@ -537,7 +537,7 @@ static int launch_dw(psc_ctx* ctx, const DwArgs& P, dim3 grid, size_t smem, cuda
 
 template <int NT8>
 static int launch_dx(psc_ctx* ctx, const DxArgs& P, dim3 grid, size_t smem, cudaStream_t st) {
-  PSC_CUDA(ctx, cudaFuncSetAttribute(k_conv_dx<NT8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  PSC_CUDA(ctx, psc_smem_optin(k_conv_dx<NT8>));
   k_conv_dx<NT8><<<grid, CBW_NT, smem, st>>>(P);
   PSC_LAUNCH_CHECK(ctx);
   return 0;

@@ -313,7 +313,7 @@ int psc_conv_tc_forward(psc_ctx* ctx, const ConvGeom& g, const __nv_bfloat16* a,
   k_conv_wt<<<std::min(148 * 4, psc_div_up((long)N * Kpad, 256)), 256, 0, st>>>(w, K, g.Cout, N, Kpad, wt);
   PSC_LAUNCH_CHECK(ctx);
   const size_t smem = CT_NS * (size_t)(CT_ATILE + N * 128) + 1024;   // at most 193 KB (N = 256)
-  PSC_CUDA(ctx, cudaFuncSetAttribute(k_conv_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  PSC_CUDA(ctx, psc_smem_optin(k_conv_tc));
   const long nvo = (long)g.nxo * g.nyo * g.nzo;
   k_conv_tc<<<psc_div_up(nvo, CT_M), CT_NT, smem, st>>>(a, s, wt, bias, g, Kpad, N, act, o, out32,
                                                        ctx->wait_limit, ctx->dev_status);

@@ -411,7 +411,7 @@ int psc_chol_inv_dev(psc_ctx* ctx, double* S, int k, double* X, cudaStream_t st)
   const size_t dyn = chol_inv_smem_doubles(k) * sizeof(double);
   if (dyn <= 200 * 1024) {
     if (dyn > 48 * 1024)
-      PSC_CUDA(ctx, cudaFuncSetAttribute(k_chol_inv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+      PSC_CUDA(ctx, psc_smem_optin(k_chol_inv));
     k_chol_inv<<<1, CI_NT, dyn, st>>>(S, k, X, ctx->dev_status);
     PSC_LAUNCH_CHECK(ctx);
     return 0;
@@ -419,8 +419,8 @@ int psc_chol_inv_dev(psc_ctx* ctx, double* S, int k, double* X, cudaStream_t st)
   double* D = X;   // R11^{-T} of the current block step, in the first CB x CB of X (overwritten below)
   const int psmem = (CB + 64) * (CB + 1) * (int)sizeof(double);
   const int usmem = 2 * CB * (64 + 1) * (int)sizeof(double);
-  PSC_CUDA(ctx, cudaFuncSetAttribute(k_potrf_panel, cudaFuncAttributeMaxDynamicSharedMemorySize, psmem));
-  PSC_CUDA(ctx, cudaFuncSetAttribute(k_potrf_update, cudaFuncAttributeMaxDynamicSharedMemorySize, usmem));
+  PSC_CUDA(ctx, psc_smem_optin(k_potrf_panel));
+  PSC_CUDA(ctx, psc_smem_optin(k_potrf_update));
   for (int j0 = 0; j0 < k; j0 += CB) {
     const int nb = std::min(CB, k - j0);
     k_potrf_diag<<<1, 256, 0, st>>>(S, k, j0, D, ctx->dev_status);
@@ -441,7 +441,7 @@ int psc_chol_inv_dev(psc_ctx* ctx, double* S, int k, double* X, cudaStream_t st)
   const size_t tdyn = ((size_t)(8 + ch) * k + ch) * sizeof(double);
   PSC_REQUIRE(ctx, tdyn <= 227 * 1024, "chol_inv: k too large for the triangular inverse");
   if (tdyn > 48 * 1024)
-    PSC_CUDA(ctx, cudaFuncSetAttribute(k_trtri_warp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tdyn));
+    PSC_CUDA(ctx, psc_smem_optin(k_trtri_warp));
   k_trtri_warp<<<psc_div_up(k, 8), 256, tdyn, st>>>(S, k, ch, X);
   PSC_LAUNCH_CHECK(ctx);
   return 0;
@@ -785,11 +785,11 @@ int psc_syev_impl(psc_ctx* ctx, double* A, int k, double* evals, double* evecs, 
 #define PSC_SYTRD(NTH)                                                                                      \
   {                                                                                                         \
     if (dyn > 48 * 1024)                                                                                    \
-      PSC_CUDA(ctx, cudaFuncSetAttribute(k_sytrd<NTH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn)); \
+      PSC_CUDA(ctx, psc_smem_optin(k_sytrd<NTH>)); \
     k_sytrd<NTH><<<1, NTH, dyn, st>>>(A, k, on_chip ? 1 : 0, hv, ab, tau);                                  \
   }
   if (clustered) {
-    PSC_CUDA(ctx, cudaFuncSetAttribute(k_sytrd_cl, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn_cl));
+    PSC_CUDA(ctx, psc_smem_optin(k_sytrd_cl));
     k_sytrd_cl<<<SY_CL, SY_CNT, dyn_cl, st>>>(A, k, hv, ab, tau);
   } else if (!on_chip) PSC_SYTRD(1024)
   else if (k <= 96) PSC_SYTRD(256)
@@ -800,7 +800,7 @@ int psc_syev_impl(psc_ctx* ctx, double* A, int k, double* evals, double* evecs, 
   if (rc) return rc;
   const size_t dyn2 = ormtr_smem_bytes(k);
   if (dyn2 > 48 * 1024)
-    PSC_CUDA(ctx, cudaFuncSetAttribute(k_ormtr, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn2));
+    PSC_CUDA(ctx, psc_smem_optin(k_ormtr));
   k_ormtr<<<psc_div_up(k, OR_NW), OR_NW * 32, dyn2, st>>>(hv, tau, k, Z, evecs);
   PSC_LAUNCH_CHECK(ctx);
   return 0;

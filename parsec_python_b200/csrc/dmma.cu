@@ -261,11 +261,11 @@ int psc_gram_pair_dmma(psc_ctx* ctx, int dtype, const void* W, const void* V, lo
   const size_t smem = 3 * (size_t)GT * GP * sizeof(double);
   dim3 grid(npair, nchunk);
   if (dtype == PSC_F64) {
-    PSC_CUDA(ctx, cudaFuncSetAttribute(k_gram_dmma<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    PSC_CUDA(ctx, psc_smem_optin(k_gram_dmma<double>));
     k_gram_dmma<double><<<grid, GNT, smem, st>>>((const double*)W, (const double*)V, ld, k, n, chunk,
                                                   (const int2*)ctx->dm_pairs, partS, partK);
   } else {
-    PSC_CUDA(ctx, cudaFuncSetAttribute(k_gram_dmma<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    PSC_CUDA(ctx, psc_smem_optin(k_gram_dmma<float>));
     k_gram_dmma<float><<<grid, GNT, smem, st>>>((const float*)W, (const float*)V, ld, k, n, chunk,
                                                  (const int2*)ctx->dm_pairs, partS, partK);
   }
@@ -283,10 +283,10 @@ int psc_gemm_tall_dmma(psc_ctx* ctx, int dtype, const void* W, long ldw, int k, 
   dim3 grid(psc_div_up(kout, MC), psc_div_up(ctx->n, MR));
   PSC_REQUIRE(ctx, grid.y <= 65535u, "gemm: too many row blocks");
   if (dtype == PSC_F64) {
-    PSC_CUDA(ctx, cudaFuncSetAttribute(k_gemm_dmma<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    PSC_CUDA(ctx, psc_smem_optin(k_gemm_dmma<double>));
     k_gemm_dmma<double><<<grid, GNT, smem, st>>>((const double*)W, ldw, k, Tm, kout, (double*)O, ldo, ctx->n);
   } else {
-    PSC_CUDA(ctx, cudaFuncSetAttribute(k_gemm_dmma<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    PSC_CUDA(ctx, psc_smem_optin(k_gemm_dmma<float>));
     k_gemm_dmma<float><<<grid, GNT, smem, st>>>((const float*)W, ldw, k, Tm, kout, (float*)O, ldo, ctx->n);
   }
   PSC_LAUNCH_CHECK(ctx);

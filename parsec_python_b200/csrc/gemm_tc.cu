@@ -343,7 +343,7 @@ int psc_gemm_tall_tc(psc_ctx* ctx, const float* W, long ld, int k, const double*
   PSC_LAUNCH_CHECK(ctx);
   const size_t buf_bytes = 2 * (size_t)GT_A_BYTES + 2 * (size_t)ntot * GT_KS * 4;
   const size_t smem = 2 * buf_bytes + 1024;
-  PSC_CUDA(ctx, cudaFuncSetAttribute(k_gemm_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  PSC_CUDA(ctx, psc_smem_optin(k_gemm_tc));
   k_gemm_tc<<<psc_div_up(n, GT_M), GT_NT, smem, st>>>(W, ld, k, n, ctx->tsplit, kout, ntot, n0, n1, nstage, O, ldo,
                                                       ctx->wait_limit, ctx->dev_status);
   PSC_LAUNCH_CHECK(ctx);

@@ -417,7 +417,7 @@ int psc_gram_pair_tc(psc_ctx* ctx, const float* W, const float* V, long ld, int 
     ctx->tc_pairs_k = k;
   }
   const size_t smem = 2 * (size_t)BUF_BYTES + 1024;
-  PSC_CUDA(ctx, cudaFuncSetAttribute(k_gram_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  PSC_CUDA(ctx, psc_smem_optin(k_gram_tc));
   double* dpart = reinterpret_cast<double*>(ctx->tc_part + tile_floats);
   k_gram_tc<<<dim3(npair, nchunk), TC_NT, smem, st>>>(W, V, ld, k, n, chunk, (const int2*)ctx->tc_pairs,
                                                       ctx->tc_part, dpart, ctx->wait_limit, ctx->dev_status);

@@ -508,7 +508,7 @@ k_tri_invit(const double* __restrict__ ab, int k, const double* __restrict__ eva
 }
 
 static int tri_smem(psc_ctx* ctx, const void* func, size_t bytes) {
-  if (bytes > 48 * 1024) PSC_CUDA(ctx, cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  if (bytes > 48 * 1024) PSC_CUDA(ctx, psc_smem_optin(func));
   return 0;
 }
 

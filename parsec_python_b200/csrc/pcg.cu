@@ -229,8 +229,7 @@ static int cg_iterations(psc_ctx* ctx, int count, cudaStream_t st) {
 #define PSC_CG_A(RR)                                                                                     \
   if (ctx->radius == RR) {                                                                               \
     if (pl.smem > 40 * 1024)                                                                             \
-      PSC_CUDA(ctx, cudaFuncSetAttribute(k_cg_dir_stencil<RR>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                                         (int)pl.smem));                                                 \
+      PSC_CUDA(ctx, psc_smem_optin(k_cg_dir_stencil<RR>, 96));                                                 \
     k_cg_dir_stencil<RR><<<pl.grid, CG_NT, pl.smem, st>>>(ctx->cg_r, pold, pnew, ctx->cg_ap, ctx->nx, ctx->ny, \
                                                           ctx->nz, ctx->lap_c0, cw, ctx->scalars, ctx->cg_ro,  \
                                                           part2, PSC_RED_BLOCKS, part1);                 \

@@ -467,15 +467,15 @@ static int spec_apply(psc_ctx* ctx, double* r, double* z, const double* sc, doub
   double* t = ctx->spec_tmp;
   const int xy_smem = (int)(((size_t)P.rows * P.pd +
                              2 * std::max((size_t)P.X.kp * P.X.pm, (size_t)P.Y.kp * P.Y.pm)) * sizeof(double));
-  PSC_CUDA(ctx, cudaFuncSetAttribute(k_spec_xy<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, xy_smem));
-  PSC_CUDA(ctx, cudaFuncSetAttribute(k_spec_xy<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, xy_smem));
+  PSC_CUDA(ctx, psc_smem_optin(k_spec_xy<true>));
+  PSC_CUDA(ctx, psc_smem_optin(k_spec_xy<false>));
   P.in = r;
   P.out = t;
   k_spec_xy<true><<<ctx->nz, XY_NT, xy_smem, st>>>(P);
   PSC_LAUNCH_CHECK(ctx);
   const int zrows = std::max(8 * ((ctx->nz + 7) / 8), Z.kp);
   const int z_smem = (int)(((size_t)zrows * Z_P + 2 * (size_t)Z.kp * Z.pm) * sizeof(double));
-  PSC_CUDA(ctx, cudaFuncSetAttribute(k_spec_z, cudaFuncAttributeMaxDynamicSharedMemorySize, z_smem));
+  PSC_CUDA(ctx, psc_smem_optin(k_spec_z));
   k_spec_z<<<psc_div_up((long)ctx->nx * ctx->ny, Z_W), Z_NT, z_smem, st>>>(t, t, P.X, P.Y, Z, zrows, sc);
   PSC_LAUNCH_CHECK(ctx);
   P.in = t;

@@ -260,6 +260,18 @@ void psc_note_launch();
     }                                                                                  \
   } while (0)
 
+// Dynamic shared memory beyond 48 KB has to be allowed for a kernel, and the
+// limit is the kernel's, for every thread of the process: it is always set to
+// the same size, the 227 KB that an SM gives one CTA less what the kernel's
+// static arrays may take (1 KB; exact where calls go up to the limit).  With
+// each call's own size, one host thread could lower the limit between another's
+// setting and its launch.
+template <typename K>
+inline cudaError_t psc_smem_optin(K kernel, int static_bytes = 1024) {
+  return cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              227 * 1024 - static_bytes);
+}
+
 static inline int psc_div_up(long a, long b) { return (int)((a + b - 1) / b); }
 
 // ---------------------------------------------------------------------------

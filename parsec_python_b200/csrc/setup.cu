@@ -387,7 +387,7 @@ extern "C" int psc_sad_setup(psc_ctx* ctx, int natoms, const int* species, const
     smem = std::max(smem, b);
   }
   if (fits && smem <= ST_SMEM_MAX) {
-    PSC_CUDA(ctx, cudaFuncSetAttribute(k_sad_tab, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    PSC_CUDA(ctx, psc_smem_optin(k_sad_tab));
     k_sad_tab<<<psc_div_up(ctx->n, ST_NT * ST_P), ST_NT, smem, st>>>(ctx->nx, ctx->ny, ctx->nz, ctx->h, radius, natoms,
                                                                     sp_d, xyz_d, tab, h3, fourpi, rho0, hpot0, ppot);
   } else {

@@ -158,7 +158,7 @@ static int launch_stencil_t(psc_ctx* ctx, const StencilPlan& p, const T* X, long
                             cudaStream_t st) {
   auto kern = k_stencil<T, R, PPT>;
   if (p.smem > 40 * 1024) {
-    PSC_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem));
+    PSC_CUDA(ctx, psc_smem_optin(kern, 64));
   }
   kern<<<p.grid, 256, p.smem, st>>>(X, ldx, P, ldp, Y, ldy, pot, ctx->nx, ctx->ny, ctx->nz, p.zchunk, w,
                                     coef, a, b, g, dot_partial, active);

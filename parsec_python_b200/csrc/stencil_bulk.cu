@@ -259,7 +259,7 @@ static int launch_bulk(psc_ctx* ctx, const BulkArgs<T>& A0, int k, cudaStream_t 
   A.sched = psc_stencil_sched(ctx, nslab, k, R + 6, 2 * sms, &nwork, st);
   PSC_REQUIRE(ctx, A.sched != nullptr, "stencil: work table allocation failed");
   auto kern = k_stencil_bulk<T, R, PPT>;
-  PSC_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  PSC_CUDA(ctx, psc_smem_optin(kern));
   kern<<<nwork, BNT, smem, st>>>(A);
   PSC_LAUNCH_CHECK(ctx);
   return 0;

@@ -819,7 +819,7 @@ const int4* psc_stencil_sched(psc_ctx* ctx, int nslab, int k, int fill, int slot
 template <typename T, int R, int YA, int VW, bool PK, bool HASP, bool HASV, int DEEP>
 static int launch_tma_k(psc_ctx* ctx, const TmaArgs<T>& A, int nwork, size_t smem, cudaStream_t st) {
   auto kern = k_stencil_tma<T, R, YA, VW, PK, HASP, HASV, DEEP>;
-  PSC_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  PSC_CUDA(ctx, psc_smem_optin(kern));
   kern<<<nwork, TNT, smem, st>>>(A);
   PSC_LAUNCH_CHECK(ctx);
   return 0;

@@ -413,7 +413,7 @@ extern "C" int psc_conv3d_fwd(psc_ctx* ctx, const int* geom, const void* A, cons
     const int aligned = ((reinterpret_cast<uintptr_t>(o) | reinterpret_cast<uintptr_t>(out32)) & 15) == 0;
     const dim3 grid(nbx * nby * nbz, g.Cout / 8);
     auto kern = g.ksize == 3 ? k_conv_fwd8<3> : k_conv_fwd8<1>;
-    PSC_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    PSC_CUDA(ctx, psc_smem_optin(kern));
     kern<<<grid, FWD_NT, smem, st>>>(a, s, w, bias, g, act, nbx, nby, aligned, o, out32);
   } else if (g.Cout % 16 == 0) {
     dim3 grid(psc_div_up(nvo, FWD_NT), g.Cout / 16);
