@@ -124,8 +124,9 @@ k_conv_fwd(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict_
 // multiply-adds and reads the input 27 times through L1 (852 us for the three
 // layers of a 90^3 pass); this one takes 456 us and is bound by the FP32 pipe.  Every output adds its terms in k_conv_fwd<8>'s order (32
 // input channels at a time, taps, channels), so the results are the same
-// bits; a tap outside the grid adds a zero product instead of being skipped
-// (as in the tensor-core kernel).
+// bits.  A tap outside the grid adds a zero product here, which an infinite or
+// NaN weight would turn into NaN: a thread that ends with a NaN takes its
+// voxels' sums again without those taps (conv_fwd_point; 0.8 % of a 90^3 pass).
 // ---------------------------------------------------------------------------
 constexpr int F8_X = 32, F8_Y = 4, F8_Z = 4;   // voxels per CTA (128 threads)
 
@@ -177,6 +178,30 @@ __device__ __forceinline__ void fwd8_chunk(const uint4* x, int hx, int hxy, int 
   }
 }
 
+// One output before the activation, taps outside the grid skipped; a sum that
+// has become NaN stays one.
+__device__ __noinline__ float conv_fwd_point(const __nv_bfloat16* A, const __nv_bfloat16* S, const __nv_bfloat16* W,
+                                             float sum, const ConvGeom& g, int x, int y, int z, int co) {
+  const int pad = g.ksize / 2, taps = g.ksize * g.ksize * g.ksize;
+  for (int cc = 0; cc < g.Cin; cc += WTILE / 8) {
+    const int cn = min(WTILE / 8, g.Cin - cc);
+    for (int tap = 0; tap < taps; ++tap) {
+      const int xi = x + tap % g.ksize - pad, yi = y + (tap / g.ksize) % g.ksize - pad,
+                zi = z + tap / (g.ksize * g.ksize) - pad;
+      if (xi < 0 || yi < 0 || zi < 0 || xi >= g.nxi || yi >= g.nyi || zi >= g.nzi) continue;
+      for (int c = 0; c < cn; c += 8) {
+        float v[8];
+        unpack8(conv_vin8(A, S, g, xi, yi, zi, cc + c), v);
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          sum = fmaf(v[j], __bfloat162float(W[((long)tap * g.Cin + cc + c + j) * g.Cout + co]), sum);
+      }
+      if (sum != sum) return sum;
+    }
+  }
+  return sum;
+}
+
 template <int KS>
 __global__ void __launch_bounds__(FWD_NT)
 k_conv_fwd8(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict__ S,
@@ -223,6 +248,24 @@ k_conv_fwd8(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict
   }
   const int y = y0 + ty, z = z0 + tz;
   if (y >= g.nyo || z >= g.nzo) return;
+  bool nan = false;
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int p = 0; p < 4; ++p) nan |= acc[i][p].x != acc[i][p].x || acc[i][p].y != acc[i][p].y;
+  if (nan) {
+#pragma unroll 1
+    for (int e = 0; e < 4 * 8; ++e) {
+      const int x = x0 + tx + 8 * (e >> 3), co = co0 + (e & 7);
+      if (x >= g.nxo) break;
+      const float a = conv_fwd_point(A, S, W, bias[co], g, x, y, z, co);
+      const float v = act == 1 ? fmaxf(a, 0.0f) : (act == 2 ? (a > 0.0f ? a : LEAK * a) : a);
+      const long q = (x + (long)g.nxo * (y + (long)g.nyo * z)) * g.Cout + co;
+      out[q] = __float2bfloat16_rn(v);
+      if (out32) out32[q] = v;
+    }
+    return;
+  }
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int x = x0 + tx + 8 * i;
