@@ -342,8 +342,8 @@ int psc_set_conv_impl(psc_ctx* ctx, int impl);
 /* act: 0 identity, 1 ReLU, 2 leaky ReLU (slope 1/16 below zero).
  * Backward of one convolution.  gout: dL/d(out) FP32 [nvo][Cout]; out: the
  * forward's BF16 output (needed when act != 0);
- * gm: FP32 scratch [nvo][Cout] (may alias gout; contents unspecified); dvin: FP32 scratch
- * [nvi][Ca+Cs] or NULL to skip the input gradient; dA / dS: FP32 gradients of
+ * gm: FP32 [nvo][Cout], receives the gradient through the activation (may
+ * alias gout); dvin: FP32 scratch [nvi][Ca+Cs] or NULL to skip the input gradient; dA / dS: FP32 gradients of
  * A and S, overwritten (acc = 0) or accumulated (acc = 1), NULL to skip; dW,
  * dB: FP32 weight and bias gradients (overwritten); work: FP32 scratch of
  * work_floats (>= chunks x 27 Cin Cout). */

@@ -3,10 +3,13 @@
 // dispatches here).
 //
 // Both products contract an FP32 gradient with BF16 data, and the gradient
-// must not lose bits.  So the gradient is written once as three BF16 planes
-// hi + mid + lo that add up to it exactly (8 significant bits each, split by
-// truncation), and every product is three mma.sync.m16n8k16 (BF16 operands,
-// FP32 accumulate) from the smallest plane up.  The tensor core's FP32
+// must not lose bits.  So a brick of the gradient is staged as three BF16
+// planes hi + mid + lo of 8 significant bits each, split by truncation (exact
+// from 2^-110 up; below, bits under BF16's smallest subnormal, 2^-133, are
+// cut), and every product is three mma.sync.m16n8k16 (BF16 operands, FP32
+// accumulate) from the smallest plane up.  The split is made again for every
+// brick: a pass that wrote the planes once needed 6 bytes per entry of context
+// memory that overlapping calls shared and a stream capture could not allocate.  The tensor core's FP32
 // accumulation does not round to nearest, so no accumulator runs through it
 // for long: after the three MMAs of one 16-entry step the result is added to
 // a register accumulator by an ordinary FP32 add (four adds per three MMAs).
@@ -14,8 +17,8 @@
 // that rate; its truncation over thousands of steps would cost 2e-5 of a
 // gradient, 30 times this path's error.)
 //
-//   k_conv_prep  gradient through the activation, split into the planes, and
-//                the bias gradient's partial sums: one pass over the gradient
+//   k_conv_prep  gradient through the activation into gm, and the bias
+//                gradient's partial sums: one pass over the gradient
 //   k_conv_dw    dW[tap][ci][co] = sum_v X[v s + tap - pad][ci] G[v][co].  A
 //                CTA stages a brick of 8 x 4 x 4 output voxels: the input
 //                with its halo once for all the taps (16 bytes = 8 channels
@@ -94,35 +97,55 @@ __device__ __forceinline__ uint4 load8(const __nv_bfloat16* p, int aligned) {
   return make_uint4(w[0], w[1], w[2], w[3]);
 }
 
-// x = hi + mid + lo exactly, each with 8 significant bits (BF16 bit patterns
-// in the upper halves); an infinity or NaN stays in hi alone
-__device__ __forceinline__ void split3(float x, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
-  const uint32_t b = __float_as_uint(x);
-  hi = b & 0xffff0000u;
-  if ((b & 0x7f800000u) == 0x7f800000u) {
-    if ((b & 0x007fffffu) && !(hi & 0x007fffffu)) hi |= 0x00400000u;   // keep a NaN a NaN
-    mid = lo = 0u;
-    return;
+// 8 FP32 values, whatever the alignment of p
+__device__ __forceinline__ void load8f(const float* p, int aligned, float (&x)[8]) {
+  if (aligned) {
+    const float4 a = __ldg(reinterpret_cast<const float4*>(p)), b = __ldg(reinterpret_cast<const float4*>(p) + 1);
+    x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w;
+    x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
+  } else {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) x[j] = p[j];
   }
-  const float r = x - __uint_as_float(hi);
-  mid = __float_as_uint(r) & 0xffff0000u;
-  lo = __float_as_uint(r - __uint_as_float(mid)) & 0xffff0000u;
+}
+
+// x - (its upper half); nothing is left of an infinity or a NaN
+__device__ __forceinline__ float split_rest(float x) {
+  const uint32_t b = __float_as_uint(x);
+  return (b & 0x7f800000u) == 0x7f800000u ? 0.0f : x - __uint_as_float(b & 0xffff0000u);
+}
+
+// x = hi + mid + lo: the upper half of x's bits, of the rest's, and of what
+// is left, two values to a word
+__device__ __forceinline__ void split8(const float (&x)[8], uint4 (&plane)[3]) {
+  uint32_t w[3][4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    float a = x[2 * j], b = x[2 * j + 1];
+#pragma unroll
+    for (int t = 0; t < 3; ++t) {
+      w[t][j] = __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
+      a = split_rest(a);
+      b = split_rest(b);
+    }
+  }
+#pragma unroll
+  for (int t = 0; t < 3; ++t) plane[t] = make_uint4(w[t][0], w[t][1], w[t][2], w[t][3]);
 }
 }  // namespace
 
-// Planes [3][nvo][Cout] of gm = gout act'(out), and part[CTA][Cout] = sums of
-// gm over the CTA's voxels.  A thread owns one octet of channels and every
-// R-th voxel of the CTA's range; the rows are added in order.
+// gm = gout act'(out) (gm may be gout), and part[CTA][Cout] = sums of gm over
+// the CTA's voxels.  A thread owns one octet of channels and every R-th voxel
+// of the CTA's range; the rows are added in order.
 __global__ void __launch_bounds__(256)
-k_conv_prep(const float* __restrict__ gout, const __nv_bfloat16* __restrict__ out, long nvo, int Cout, int act,
-            int aligned, uint4* __restrict__ planes, long vchunk, float* __restrict__ part) {
+k_conv_prep(const float* gout, const __nv_bfloat16* __restrict__ out, long nvo, int Cout, int act, int aligned,
+            float* gm, long vchunk, float* __restrict__ part) {
   __shared__ float sh[256 * 8];
   const int oct = Cout / 8;
   const int R = 256 / oct;
   const int o = threadIdx.x % oct, r = threadIdx.x / oct;
   const long v0 = (long)blockIdx.x * vchunk, v1 = min(nvo, v0 + vchunk);
   const float below = act == 2 ? CB_LEAK : 0.0f;
-  const long plane = nvo * oct;
   float s[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) s[j] = 0.0f;
@@ -148,18 +171,16 @@ k_conv_prep(const float* __restrict__ gout, const __nv_bfloat16* __restrict__ ou
           if (!(y > 0.0f)) x[j] *= below;
         }
       }
-      uint32_t q[3][4];
+      if (act != 0 || gm != gout) {
+        if (aligned) {
+          float4* gp = reinterpret_cast<float4*>(gm) + 2 * e;
+          gp[0] = make_float4(x[0], x[1], x[2], x[3]);
+          gp[1] = make_float4(x[4], x[5], x[6], x[7]);
+        } else {
 #pragma unroll
-      for (int j = 0; j < 8; j += 2) {
-        uint32_t h0, m0, l0, h1, m1, l1;
-        split3(x[j], h0, m0, l0);
-        split3(x[j + 1], h1, m1, l1);
-        q[0][j >> 1] = (h0 >> 16) | h1;
-        q[1][j >> 1] = (m0 >> 16) | m1;
-        q[2][j >> 1] = (l0 >> 16) | l1;
+          for (int j = 0; j < 8; ++j) gm[8 * e + j] = x[j];
+        }
       }
-#pragma unroll
-      for (int t = 0; t < 3; ++t) planes[t * plane + e] = make_uint4(q[t][0], q[t][1], q[t][2], q[t][3]);
 #pragma unroll
       for (int j = 0; j < 8; ++j) s[j] += x[j];
     }
@@ -186,7 +207,8 @@ __global__ void k_conv_bias(const float* __restrict__ part, int np, int Cout, fl
 struct DwArgs {
   const __nv_bfloat16* A;
   const __nv_bfloat16* S;
-  const uint4* planes;
+  const float* G;         // gradient through the activation [nvo][Cout]
+  int g_aligned;          // G is 16-byte aligned
   ConvGeom g;
   int nbx, nby, nbz;      // bricks per axis
   int bricks_per_chunk;
@@ -237,7 +259,6 @@ k_conv_dw(DwArgs P) {
 
   const int nb = P.nbx * P.nby * P.nbz;
   const int b0 = blockIdx.x * P.bricks_per_chunk, b1 = min(nb, b0 + P.bricks_per_chunk);
-  const long nvo = (long)g.nxo * g.nyo * g.nzo;
   const int oct = g.Cout / 8;
   const uint4 zero4 = make_uint4(0u, 0u, 0u, 0u);
   for (int b = b0; b < b1; ++b) {
@@ -267,9 +288,14 @@ k_conv_dw(DwArgs P) {
         if (v >= BV) break;
         const int x = bx + v % BX, y = by + (v / BX) % BY, z = bz + v / (BX * BY);
         const bool in = x < g.nxo && y < g.nyo && z < g.nzo && n0 / 8 + j < oct;
-        const uint4* src = P.planes + (x + (long)g.nxo * (y + (long)g.nyo * z)) * oct + n0 / 8 + j;
+        uint4 pl[3] = {zero4, zero4, zero4};
+        if (in) {
+          float gv[8];
+          load8f(P.G + (x + (long)g.nxo * (y + (long)g.nyo * z)) * g.Cout + n0 + 8 * j, P.g_aligned, gv);
+          split8(gv, pl);
+        }
 #pragma unroll
-        for (int t = 0; t < 3; ++t) Gs[(t * NT8 + j) * BV + v] = in ? src[t * nvo * oct] : zero4;
+        for (int t = 0; t < 3; ++t) Gs[(t * NT8 + j) * BV + v] = pl[t];
       }
     }
     __syncthreads();
@@ -333,7 +359,8 @@ k_conv_dw(DwArgs P) {
 }
 
 struct DxArgs {
-  const uint4* planes;
+  const float* G;
+  int g_aligned;
   const __nv_bfloat16* W;
   ConvGeom g;
   int nbx, nby, nbz;   // bricks per axis of the coarse (class) grid
@@ -384,7 +411,6 @@ k_conv_dx(DxArgs P) {
   __syncthreads();
   const int nt = s_nt;
   const int units = nt * co8, usteps = (units + 1) / 2;
-  const long nvo = (long)g.nxo * g.nyo * g.nzo;
   const int oct = g.Cout / 8;
   const uint4 zero4 = make_uint4(0u, 0u, 0u, 0u);
   const uint32_t gbase = smem_u32(Gs), wbase = smem_u32(Ws);
@@ -404,7 +430,7 @@ k_conv_dx(DxArgs P) {
       for (int q = 0; q < 4; ++q) acc[i][j][q] = 0.0f;
 
   // the brick voxels this thread stages (the same for every group of output
-  // channels): offsets into a plane, -1 outside the grid
+  // channels): offsets into the gradient, -1 outside the grid
   const int lco = co8 - 1;   // log2 of co8 (1 or 2)
   const int sc = threadIdx.x & lco, sw = threadIdx.x >> lco;
   long goff[5];
@@ -413,7 +439,7 @@ k_conv_dx(DxArgs P) {
     const int w = sw + q * (CBW_NT >> lco);
     const int x = cx - 1 + w % (DX + 2), y = cy - 1 + (w / (DX + 2)) % (DY + 2), z = cz - 1 + w / ((DX + 2) * (DY + 2));
     const bool in = w < DH && x >= 0 && y >= 0 && z >= 0 && x < g.nxo && y < g.nyo && z < g.nzo;
-    goff[q] = in ? (x + (long)g.nxo * (y + (long)g.nyo * z)) * oct + sc : -1;
+    goff[q] = in ? (x + (long)g.nxo * (y + (long)g.nyo * z)) * g.Cout + 8 * sc : -1;
   }
   for (int o0 = 0; o0 < oct; o0 += co8) {
     __syncthreads();
@@ -422,9 +448,14 @@ k_conv_dx(DxArgs P) {
       const int w = sw + q * (CBW_NT >> lco);
       if (w >= DH) break;
       const bool in = goff[q] >= 0 && o0 + sc < oct;
+      uint4 pl[3] = {zero4, zero4, zero4};
+      if (in) {
+        float gv[8];
+        load8f(P.G + goff[q] + 8 * o0, P.g_aligned, gv);
+        split8(gv, pl);
+      }
 #pragma unroll
-      for (int t = 0; t < 3; ++t)
-        Gs[(t * co8 + sc) * DH + w] = in ? P.planes[t * nvo * oct + goff[q] + o0] : zero4;
+      for (int t = 0; t < 3; ++t) Gs[(t * co8 + sc) * DH + w] = pl[t];
     }
     for (int e = threadIdx.x; e < 2 * usteps * NC; e += CBW_NT) {
       const int c = e & lco, n = (e >> lco) % NC, k = (e >> lco) / NC;   // unit k co8 + c
@@ -543,32 +574,24 @@ static int launch_dx(psc_ctx* ctx, const DxArgs& P, dim3 grid, size_t smem, cuda
   return 0;
 }
 
-// Gradient through the activation as planes in ctx->conv_g3, bias gradient dB
-// and weight gradient dW; `work` holds the partial sums.
+// Gradient through the activation into gm, bias gradient dB and weight
+// gradient dW; `work` holds the partial sums.
 int psc_conv_bwd_weights(psc_ctx* ctx, const ConvGeom& g, const __nv_bfloat16* a, const __nv_bfloat16* s,
-                         const float* gout, const __nv_bfloat16* out, int act, float* dW, float* dB, float* work,
-                         long work_floats, cudaStream_t st) {
+                         const float* gout, const __nv_bfloat16* out, int act, float* gm, float* dW, float* dB,
+                         float* work, long work_floats, cudaStream_t st) {
   const int taps = g.ksize * g.ksize * g.ksize;
   const long nvo = (long)g.nxo * g.nyo * g.nzo;
   const long nw = (long)taps * g.Cin * g.Cout;
   PSC_REQUIRE(ctx, nw <= work_floats, "conv3d_bwd: work buffer too small");
-  const size_t need = 3 * (size_t)nvo * g.Cout * sizeof(__nv_bfloat16);
-  if (ctx->conv_g3_bytes < need) {
-    psc_dfree(ctx->conv_g3);
-    ctx->conv_g3 = nullptr;
-    ctx->conv_g3_bytes = 0;
-    PSC_CUDA(ctx, psc_dmalloc(&ctx->conv_g3, need));
-    ctx->conv_g3_bytes = need;
-  }
-  auto* planes = static_cast<uint4*>(ctx->conv_g3);
   {
     const int rows = 256 / (g.Cout / 8);
     long nb = std::max<long>(1, std::min<long>(148 * 4, nvo / (4 * rows)));
     nb = std::max<long>(1, std::min<long>(nb, work_floats / g.Cout));
     const long vchunk = (nvo + nb - 1) / nb;
     nb = (nvo + vchunk - 1) / vchunk;
-    const int aligned = ((reinterpret_cast<uintptr_t>(gout) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
-    k_conv_prep<<<(int)nb, 256, 0, st>>>(gout, out, nvo, g.Cout, act, aligned, planes, vchunk, work);
+    const int aligned = ((reinterpret_cast<uintptr_t>(gout) | reinterpret_cast<uintptr_t>(gm) |
+                          reinterpret_cast<uintptr_t>(out)) & 15) == 0;
+    k_conv_prep<<<(int)nb, 256, 0, st>>>(gout, out, nvo, g.Cout, act, aligned, gm, vchunk, work);
     PSC_LAUNCH_CHECK(ctx);
     k_conv_bias<<<psc_div_up(g.Cout, 8), 256, 0, st>>>(work, (int)nb, g.Cout, dB);
     PSC_LAUNCH_CHECK(ctx);
@@ -576,7 +599,8 @@ int psc_conv_bwd_weights(psc_ctx* ctx, const ConvGeom& g, const __nv_bfloat16* a
   const int oct = g.Cout / 8, nu = (g.Cin / 8) * taps;
   const int nt8 = oct == 1 ? 1 : (oct == 2 ? 2 : 4);
   DwArgs P;
-  P.A = a; P.S = s; P.planes = planes; P.g = g; P.part = work;
+  P.A = a; P.S = s; P.G = gm; P.g = g; P.part = work;
+  P.g_aligned = (reinterpret_cast<uintptr_t>(gm) & 15) == 0;
   P.nbx = psc_div_up(g.nxo, BX); P.nby = psc_div_up(g.nyo, BY); P.nbz = psc_div_up(g.nzo, BZ);
   P.hx = (BX - 1) * g.stride + g.ksize; P.hy = (BY - 1) * g.stride + g.ksize; P.hz = (BZ - 1) * g.stride + g.ksize;
   // units per CTA (16 MT): the split that pads least, a CTA's staging costing
@@ -616,12 +640,13 @@ int psc_conv_bwd_weights(psc_ctx* ctx, const ConvGeom& g, const __nv_bfloat16* a
   return 0;
 }
 
-// Input gradient of all Cin channels into out (ldo floats per voxel), from
-// the planes psc_conv_bwd_weights left.
-int psc_conv_bwd_input(psc_ctx* ctx, const ConvGeom& g, const __nv_bfloat16* w, float* out, int ldo, int acc,
-                       cudaStream_t st) {
+// Input gradient of all Cin channels into out (ldo floats per voxel, not
+// overlapping gm), from the gm that psc_conv_bwd_weights left.
+int psc_conv_bwd_input(psc_ctx* ctx, const ConvGeom& g, const __nv_bfloat16* w, const float* gm, float* out, int ldo,
+                       int acc, cudaStream_t st) {
   DxArgs P;
-  P.planes = static_cast<const uint4*>(ctx->conv_g3);
+  P.G = gm;
+  P.g_aligned = (reinterpret_cast<uintptr_t>(gm) & 15) == 0;
   P.W = w; P.g = g; P.out = out; P.ldo = ldo; P.acc = acc;
   P.w_aligned = (reinterpret_cast<uintptr_t>(w) & 15) == 0;
   P.o_aligned = (reinterpret_cast<uintptr_t>(out) & 7) == 0;

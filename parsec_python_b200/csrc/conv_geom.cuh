@@ -41,10 +41,11 @@ int psc_conv_tc_forward(psc_ctx* ctx, const ConvGeom& g, const __nv_bfloat16* a,
                         const __nv_bfloat16* w, const float* bias, int act, __nv_bfloat16* o, float* out32,
                         cudaStream_t st);
 
-// backward on the tensor cores (conv_bwd.cu): planes of the gradient, dW and
-// dB; then the input gradient (all Cin channels, ldo floats per voxel)
+// backward on the tensor cores (conv_bwd.cu): the gradient through the
+// activation (gm), dW and dB; then the input gradient (all Cin channels, ldo
+// floats per voxel)
 int psc_conv_bwd_weights(psc_ctx* ctx, const ConvGeom& g, const __nv_bfloat16* a, const __nv_bfloat16* s,
-                         const float* gout, const __nv_bfloat16* out, int act, float* dW, float* dB, float* work,
-                         long work_floats, cudaStream_t st);
-int psc_conv_bwd_input(psc_ctx* ctx, const ConvGeom& g, const __nv_bfloat16* w, float* out, int ldo, int acc,
-                       cudaStream_t st);
+                         const float* gout, const __nv_bfloat16* out, int act, float* gm, float* dW, float* dB,
+                         float* work, long work_floats, cudaStream_t st);
+int psc_conv_bwd_input(psc_ctx* ctx, const ConvGeom& g, const __nv_bfloat16* w, const float* gm, float* out, int ldo,
+                       int acc, cudaStream_t st);

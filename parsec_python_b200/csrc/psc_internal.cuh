@@ -145,8 +145,6 @@ struct psc_ctx {
   int conv_tc = 1;
   void* conv_wt = nullptr;       // BF16 weights transposed to [Cout rounded to 16][K rounded to 64]
   size_t conv_wt_bytes = 0;
-  void* conv_g3 = nullptr;       // output gradient of one layer as three BF16 planes (backward)
-  size_t conv_g3_bytes = 0;
   // sphere mask of the Hamiltonian (0: the whole cube): H X is zero at
   // points farther than sqrt(mask_r2) from mask_c (the cube's centre)
   double mask_r2 = 0.0;

@@ -483,13 +483,15 @@ extern "C" int psc_conv3d_bwd(psc_ctx* ctx, const int* geom, const void* A, cons
   const auto* s = static_cast<const __nv_bfloat16*>(S);
   const auto* w = static_cast<const __nv_bfloat16*>(W);
   // output gradient through the activation, weight and bias gradients
-  int rc = psc_conv_bwd_weights(ctx, g, a, s, gout, static_cast<const __nv_bfloat16*>(out), act, dW, dB, work,
+  int rc = psc_conv_bwd_weights(ctx, g, a, s, gout, static_cast<const __nv_bfloat16*>(out), act, gm, dW, dB, work,
                                 work_floats, st);
   if (rc || !dvin) return rc;
-  // input gradient: straight into dA when it is A's alone, else through dvin
-  // and split into dA and dS
-  if (!g.up && g.Cs == 0 && dA) return psc_conv_bwd_input(ctx, g, w, dA, g.Ca, acc_a, st);
-  rc = psc_conv_bwd_input(ctx, g, w, dvin, g.Cin, 0, st);
+  // input gradient: straight into dA when it is A's alone and dA lies clear of
+  // gm (which is still read), else through dvin and split into dA and dS
+  const long nvi = (long)g.nxi * g.nyi * g.nzi, nvo = (long)g.nxo * g.nyo * g.nzo;
+  const bool clear = dA + nvi * g.Ca <= gm || gm + nvo * g.Cout <= dA;
+  if (!g.up && g.Cs == 0 && dA && clear) return psc_conv_bwd_input(ctx, g, w, gm, dA, g.Ca, acc_a, st);
+  rc = psc_conv_bwd_input(ctx, g, w, gm, dvin, g.Cin, 0, st);
   if (rc) return rc;
   if (dA) {
     k_split_grad_a<<<148 * 8, 256, 0, st>>>(dvin, g, acc_a, dA);
