@@ -46,6 +46,12 @@
 // and, on the coarse levels, too few bricks for 148 SMs.  Relative errors
 // against 64 bits over the network's layers: dW 7e-8 to 9e-8, input
 // 8e-8 to 2.5e-7, bias 3e-8 to 8e-8 (before: up to 6e-7, 1e-6 and 3e-7).
+//
+// Infinities and NaNs.  The planes of an entry, the zeros staged for what lies
+// outside the grid and the padding of a brick all turn an infinite factor into
+// a NaN that the product of the two numbers would not give.  So a NaN in a
+// result only says that an infinity or a NaN was at hand: its sum is taken
+// again from the FP32 gradient, over the terms there are (dw_entry, dx_entry).
 #include "psc_internal.cuh"
 #include "../../include/psc.h"
 
@@ -109,14 +115,13 @@ __device__ __forceinline__ void load8f(const float* p, int aligned, float (&x)[8
   }
 }
 
-// x - (its upper half); nothing is left of an infinity or a NaN
+// x - (its upper half)
 __device__ __forceinline__ float split_rest(float x) {
-  const uint32_t b = __float_as_uint(x);
-  return (b & 0x7f800000u) == 0x7f800000u ? 0.0f : x - __uint_as_float(b & 0xffff0000u);
+  return x - __uint_as_float(__float_as_uint(x) & 0xffff0000u);
 }
 
 // x = hi + mid + lo: the upper half of x's bits, of the rest's, and of what
-// is left, two values to a word
+// is left, two values to a word (an infinity or NaN leaves NaNs)
 __device__ __forceinline__ void split8(const float (&x)[8], uint4 (&plane)[3]) {
   uint32_t w[3][4];
 #pragma unroll
@@ -217,9 +222,32 @@ struct DwArgs {
   float* part;
 };
 
+// One entry's sum over the bricks b0 .. b1, term by term; a sum that has become
+// NaN stays one.
+__device__ __noinline__ float dw_entry(const DwArgs& P, int tap, int ci, int co, int b0, int b1) {
+  const ConvGeom& g = P.g;
+  const int pad = g.ksize / 2;
+  const int dx = tap % g.ksize - pad, dy = (tap / g.ksize) % g.ksize - pad, dz = tap / (g.ksize * g.ksize) - pad;
+  float s = 0.0f;
+  for (int b = b0; b < b1; ++b)
+    for (int v = 0; v < BV; ++v) {
+      const int xo = (b % P.nbx) * BX + v % BX, yo = ((b / P.nbx) % P.nby) * BY + (v / BX) % BY,
+                zo = (b / (P.nbx * P.nby)) * BZ + v / (BX * BY);
+      if (xo >= g.nxo || yo >= g.nyo || zo >= g.nzo) continue;
+      const int x = xo * g.stride + dx, y = yo * g.stride + dy, z = zo * g.stride + dz;
+      if (x < 0 || y < 0 || z < 0 || x >= g.nxi || y >= g.nyi || z >= g.nzi) continue;
+      const long vs = x + (long)g.nxi * (y + (long)g.nyi * z);
+      const long va = g.up ? (x >> 1) + (long)g.nxa * ((y >> 1) + (long)g.nya * (z >> 1)) : vs;
+      const __nv_bfloat16 xv = ci < g.Ca ? P.A[va * g.Ca + ci] : P.S[vs * g.Cs + (ci - g.Ca)];
+      s = fmaf(__bfloat162float(xv), P.G[(xo + (long)g.nxo * (yo + (long)g.nyo * zo)) * g.Cout + co], s);
+      if (s != s) return s;
+    }
+  return s;
+}
+
 template <int NT8, int MT>
 __global__ void __launch_bounds__(CBW_NT)
-k_conv_dw(DwArgs P) {
+k_conv_dw(const __grid_constant__ DwArgs P) {
   extern __shared__ __align__(128) unsigned char cb_sm[];
   const ConvGeom& g = P.g;
   const int taps = g.ksize * g.ksize * g.ksize, pad = g.ksize / 2;
@@ -351,8 +379,11 @@ k_conv_dw(DwArgs P) {
       for (int j = 0; j < NT8; ++j) {
         const int co = n0 + 8 * j + 2 * (lane & 3);
         if (co < g.Cout) {
-          row[co] = acc[m][j][2 * h];
-          row[co + 1] = acc[m][j][2 * h + 1];
+          float v0 = acc[m][j][2 * h], v1 = acc[m][j][2 * h + 1];
+          if (v0 != v0) v0 = dw_entry(P, tap, ci, co, b0, b1);
+          if (v1 != v1) v1 = dw_entry(P, tap, ci, co + 1, b0, b1);
+          row[co] = v0;
+          row[co + 1] = v1;
         }
       }
     }
@@ -372,9 +403,28 @@ struct DxArgs {
   float* out;
 };
 
+// One entry of the input gradient, term by term (as dw_entry)
+__device__ __noinline__ float dx_entry(const DxArgs& P, int x, int y, int z, int ci) {
+  const ConvGeom& g = P.g;
+  const int pad = g.ksize / 2;
+  float s = 0.0f;
+  for (int tap = 0; tap < g.ksize * g.ksize * g.ksize; ++tap) {
+    const int ax = x + pad - tap % g.ksize, ay = y + pad - (tap / g.ksize) % g.ksize,
+              az = z + pad - tap / (g.ksize * g.ksize);
+    if (ax < 0 || ay < 0 || az < 0 || (g.stride == 2 && ((ax | ay | az) & 1))) continue;
+    const int xo = ax / g.stride, yo = ay / g.stride, zo = az / g.stride;
+    if (xo >= g.nxo || yo >= g.nyo || zo >= g.nzo) continue;
+    const float* gp = P.G + (xo + (long)g.nxo * (yo + (long)g.nyo * zo)) * g.Cout;
+    const __nv_bfloat16* wp = P.W + ((long)tap * g.Cin + ci) * g.Cout;
+    for (int co = 0; co < g.Cout; ++co) s = fmaf(gp[co], __bfloat162float(wp[co]), s);
+    if (s != s) return s;
+  }
+  return s;
+}
+
 template <int NT8>
 __global__ void __launch_bounds__(CBW_NT)
-k_conv_dx(DxArgs P) {
+k_conv_dx(const __grid_constant__ DxArgs P) {
   extern __shared__ __align__(128) unsigned char cb_sm[];
   const ConvGeom& g = P.g;
   constexpr int NC = NT8 * 8;
@@ -521,6 +571,8 @@ k_conv_dx(DxArgs P) {
         const int ci = ci0 + 8 * j + 2 * (lane & 3);
         if (ci >= g.Cin) continue;
         float v0 = acc[i][j][2 * h], v1 = acc[i][j][2 * h + 1];
+        if (v0 != v0) v0 = dx_entry(P, x, y, z, ci);
+        if (v1 != v1) v1 = dx_entry(P, x, y, z, ci + 1);
         if (P.o_aligned) {
           float2* p = reinterpret_cast<float2*>(row + ci);
           if (P.acc) {
