@@ -22,6 +22,7 @@
 #define PSC_RED_SLOTS 16      // simultaneous dot products per reduction launch
 #define PSC_TICKETS 1024      // arrival counters of the reductions that end in their last CTA
 #define PSC_NORM_CHUNKS 32    // row chunks of the column-norm partial sums
+#define PSC_SCHED_MASKED 0x80  // in a stencil work table's key: made for the sphere mask
 #define PSC_WAIT_DEFAULT (1L << 24)  // polls of a bounded device-side wait before it gives up
 #define PSC_DRAIN_WAIT (1L << 24)    // polls spent, after a failed wait, on copies and MMAs already issued
 

@@ -257,6 +257,7 @@ static int launch_bulk(psc_ctx* ctx, const BulkArgs<T>& A0, int k, cudaStream_t 
   int sms = 148, nwork = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
   A.sched = psc_stencil_sched(ctx, nslab, k, R + 6, 2 * sms, &nwork, st);
+  if (nwork == 0) return -1;   // no table yet, and none to be had during a stream capture
   PSC_REQUIRE(ctx, A.sched != nullptr, "stencil: work table allocation failed");
   auto kern = k_stencil_bulk<T, R, PPT>;
   PSC_CUDA(ctx, psc_smem_optin(kern));

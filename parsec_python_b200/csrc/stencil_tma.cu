@@ -784,12 +784,16 @@ static std::vector<int4> stencil_schedule_masked(const psc_ctx* ctx, int ts, int
   return comp;
 }
 
+static long long sched_key(int nslab, int k, int fill, int slots, bool masked) {
+  return ((long long)k << 32) | ((long long)nslab << 16) | ((long long)fill << 8) | (slots & 0x7f) |
+         (masked ? PSC_SCHED_MASKED : 0);
+}
+
 // Cached per context: the table of a (k, slab count, fill, mask) combination
 // is built and uploaded once.
 static const int4* stencil_sched(psc_ctx* ctx, int nslab, int k, int fill, int slots, bool masked, int ts, int* n,
                                  cudaStream_t st) {
-  const long long key = ((long long)k << 32) | ((long long)nslab << 16) | ((long long)fill << 8) | (slots & 0x7f) |
-                        (masked ? 0x80 : 0);
+  const long long key = sched_key(nslab, k, fill, slots, masked);
   for (auto& e : ctx->st_sched)
     if (e.key == key) {
       *n = e.n;
@@ -811,8 +815,17 @@ static const int4* stencil_sched(psc_ctx* ctx, int nslab, int k, int fill, int s
   return reinterpret_cast<const int4*>(b.dev);
 }
 
-// the unmasked table for another kernel with the same (column, slab, z range) items
+// The unmasked table for another kernel with the same (column, slab, z range)
+// items.  *n = 0 and NULL if it is not there yet and a capture of st forbids the
+// allocation.
 const int4* psc_stencil_sched(psc_ctx* ctx, int nslab, int k, int fill, int slots, int* n, cudaStream_t st) {
+  *n = 0;
+  const long long key = sched_key(nslab, k, fill, slots, false);
+  bool cached = false;
+  for (const auto& e : ctx->st_sched) cached = cached || e.key == key;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (!cached && (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone)) return nullptr;
+  *n = -1;
   return stencil_sched(ctx, nslab, k, fill, slots, false, 0, n, st);
 }
 
