@@ -408,10 +408,15 @@ extern "C" int psc_set_sphere_mask(psc_ctx* ctx, double radius, void* stream) {
   ctx->mask_c[1] = 0.5 * ctx->h * (ctx->ny - 1);
   ctx->mask_c[2] = 0.5 * ctx->h * (ctx->nz - 1);
   // masked work tables depend on the radius: drop the cached ones once the
-  // launches that may still read them have finished
+  // launches that may still read them have finished (the others stay, also
+  // for the captured graphs that hold them)
   PSC_CUDA(ctx, cudaStreamSynchronize((cudaStream_t)stream));
-  for (auto& e : ctx->st_sched) psc_dfree(e.dev);
-  ctx->st_sched.clear();
+  size_t keep = 0;
+  for (auto& e : ctx->st_sched) {
+    if (e.key & PSC_SCHED_MASKED) psc_dfree(e.dev);
+    else ctx->st_sched[keep++] = e;
+  }
+  ctx->st_sched.resize(keep);
   return psc_nl_apply_mask(ctx, (cudaStream_t)stream);
 }
 

@@ -58,3 +58,22 @@ def test_first_call_in_a_capture(dt):
     _apply(ctx, code, X, ref)
     _close(Y, ref)
     ctx.check_status()
+
+
+def test_captured_graph_outlives_a_sphere_mask():
+    """Setting and clearing the sphere mask leaves the tables of unmasked
+    launches where the captured graph holds them."""
+    ctx, X, Y, code = _setup("f64")
+    ref = torch.empty_like(Y)
+    _apply(ctx, code, X, ref)               # builds the table
+    graph = _capture(ctx, code, X, Y)
+    ctx.set_sphere_mask(8.0)
+    ctx.set_sphere_mask(0.0)
+    other = [_setup("f32") for _ in range(3)]   # takes freed memory, if any was
+    for c, x, y, cd in other:
+        _apply(c, cd, x, y)
+    Y.fill_(float("nan"))
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(Y, ref)
+    ctx.check_status()
