@@ -161,7 +161,6 @@ struct psc_ctx {
     long long key = 0;
     int n = 0;
     int* dev = nullptr;
-    std::vector<int> host;   // the uploaded copy (kept alive for the asynchronous upload)
   };
   std::vector<StencilSched> st_sched;
 

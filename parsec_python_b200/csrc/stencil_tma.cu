@@ -54,7 +54,6 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
-#include <cstring>
 #include <type_traits>
 #include <vector>
 
@@ -790,9 +789,9 @@ static long long sched_key(int nslab, int k, int fill, int slots, bool masked) {
 }
 
 // Cached per context: the table of a (k, slab count, fill, mask) combination
-// is built and uploaded once.
-static const int4* stencil_sched(psc_ctx* ctx, int nslab, int k, int fill, int slots, bool masked, int ts, int* n,
-                                 cudaStream_t st) {
+// is built and uploaded once.  The upload has ended before the table is handed
+// out, since the next call may be on a stream that does not wait for st.
+static const int4* stencil_sched(psc_ctx* ctx, int nslab, int k, int fill, int slots, bool masked, int ts, int* n) {
   const long long key = sched_key(nslab, k, fill, slots, masked);
   for (auto& e : ctx->st_sched)
     if (e.key == key) {
@@ -804,15 +803,16 @@ static const int4* stencil_sched(psc_ctx* ctx, int nslab, int k, int fill, int s
   std::vector<int4> tab = masked ? stencil_schedule_masked(ctx, ts, nslab, k, slots)
                                  : stencil_schedule(nslab, ctx->nz, k, fill, slots);
   e.n = (int)tab.size();
-  e.host.resize(4 * tab.size());
-  std::memcpy(e.host.data(), tab.data(), tab.size() * sizeof(int4));
   if (psc_dmalloc(&e.dev, tab.size() * sizeof(int4)) != cudaSuccess) return nullptr;
-  ctx->st_sched.push_back(std::move(e));
-  auto& b = ctx->st_sched.back();
-  if (cudaMemcpyAsync(b.dev, b.host.data(), b.host.size() * sizeof(int), cudaMemcpyHostToDevice, st) != cudaSuccess)
+  if (cudaMemcpyAsync(e.dev, tab.data(), tab.size() * sizeof(int4), cudaMemcpyHostToDevice, cudaStreamLegacy) !=
+          cudaSuccess ||
+      cudaStreamSynchronize(cudaStreamLegacy) != cudaSuccess) {
+    psc_dfree(e.dev);
     return nullptr;
-  *n = b.n;
-  return reinterpret_cast<const int4*>(b.dev);
+  }
+  ctx->st_sched.push_back(e);
+  *n = e.n;
+  return reinterpret_cast<const int4*>(e.dev);
 }
 
 // The unmasked table for another kernel with the same (column, slab, z range)
@@ -826,7 +826,7 @@ const int4* psc_stencil_sched(psc_ctx* ctx, int nslab, int k, int fill, int slot
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (!cached && (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone)) return nullptr;
   *n = -1;
-  return stencil_sched(ctx, nslab, k, fill, slots, false, 0, n, st);
+  return stencil_sched(ctx, nslab, k, fill, slots, false, 0, n);
 }
 
 template <typename T, int R, int YA, int VW, bool PK, bool HASP, bool HASV, int DEEP>
@@ -860,7 +860,7 @@ static int launch_tma_t(psc_ctx* ctx, int k, const T* X, long ldx, const T* P, l
   const int fill = R + DEEP + 2;
   int nwork = 0;
   masked = masked && ctx->mask_r2 > 0.0;
-  const int4* sched = stencil_sched(ctx, nslab, k, fill, slots, masked, TS, &nwork, st);
+  const int4* sched = stencil_sched(ctx, nslab, k, fill, slots, masked, TS, &nwork);
   PSC_REQUIRE(ctx, sched != nullptr, "stencil: work table allocation failed");
   TmaArgs<T> A;
   A.X = X; A.ldx = ldx; A.P = P; A.ldp = ldp; A.Y = Y; A.ldy = ldy; A.pot = pot;
