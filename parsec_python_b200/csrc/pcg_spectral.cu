@@ -321,9 +321,10 @@ k_spec_xy(XyArgs P) {
 }
 
 // z lines q0 .. q0 + 31 of the plane's flat (stored-mode) index: forward,
-// divide by the eigenvalue, back; in place is allowed
+// divide by the eigenvalue, back; out may be in (its solver's calls are): a CTA
+// reads all of its lines before it writes them, and no other CTA's
 __global__ void __launch_bounds__(Z_NT)
-k_spec_z(const double* __restrict__ in, double* __restrict__ out, SpecAxis X, SpecAxis Y, SpecAxis A, int rows,
+k_spec_z(const double* in, double* out, SpecAxis X, SpecAxis Y, SpecAxis A, int rows,
          const double* sc) {
   extern __shared__ double sp_sm[];
   if (sc && sc[SC_ACTIVE] == 0.0) return;
