@@ -343,10 +343,12 @@ int psc_set_conv_impl(psc_ctx* ctx, int impl);
  * Backward of one convolution.  gout: dL/d(out) FP32 [nvo][Cout]; out: the
  * forward's BF16 output (needed when act != 0);
  * gm: FP32 [nvo][Cout], receives the gradient through the activation (may
- * alias gout); dvin: FP32 scratch [nvi][Ca+Cs] or NULL to skip the input gradient; dA / dS: FP32 gradients of
- * A and S, overwritten (acc = 0) or accumulated (acc = 1), NULL to skip; dW,
- * dB: FP32 weight and bias gradients (overwritten); work: FP32 scratch of
- * work_floats (>= chunks x 27 Cin Cout). */
+ * alias gout); dvin: FP32 scratch [nvi][Ca+Cs], or NULL to skip the input
+ * gradient (any other pointer will do, dA itself for one, where up = 0, Cs = 0
+ * and dA does not overlap gm: the gradient then goes straight into dA);
+ * dA / dS: FP32 gradients of A and S, overwritten (acc = 0) or accumulated
+ * (acc = 1), NULL to skip; dW, dB: FP32 weight and bias gradients
+ * (overwritten); work: FP32 scratch of work_floats (>= chunks x 27 Cin Cout). */
 int psc_conv3d_bwd(psc_ctx* ctx, const int* geom, const void* A, const void* S, const void* W, const float* gout,
                    const void* out, int act, float* gm, float* dvin, float* dA, int acc_a, float* dS, int acc_s,
                    float* dW, float* dB, float* work, long work_floats, void* stream);

@@ -489,8 +489,8 @@ extern "C" int psc_conv3d_bwd(psc_ctx* ctx, const int* geom, const void* A, cons
   // input gradient: straight into dA when it is A's alone and dA lies clear of
   // gm (which is still read), else through dvin and split into dA and dS
   const long nvi = (long)g.nxi * g.nyi * g.nzi, nvo = (long)g.nxo * g.nyo * g.nzo;
-  const bool clear = dA + nvi * g.Ca <= gm || gm + nvo * g.Cout <= dA;
-  if (!g.up && g.Cs == 0 && dA && clear) return psc_conv_bwd_input(ctx, g, w, gm, dA, g.Ca, acc_a, st);
+  const bool clear = dA && (dA + nvi * g.Ca <= gm || gm + nvo * g.Cout <= dA);
+  if (!g.up && g.Cs == 0 && clear) return psc_conv_bwd_input(ctx, g, w, gm, dA, g.Ca, acc_a, st);
   rc = psc_conv_bwd_input(ctx, g, w, gm, dvin, g.Cin, 0, st);
   if (rc) return rc;
   if (dA) {

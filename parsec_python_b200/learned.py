@@ -197,8 +197,6 @@ class UNet3D:
             dvin = dA = dS = None
             acc_a = acc_s = 0
             if need_in:
-                nvi = self._nvox(l.skip if l.up else l.src)
-                dvin = torch.empty(nvi, l.ca + l.cs, dtype=torch.float32, device=self.dev)
                 if l.src in grads:
                     acc_a = 1
                 else:
@@ -210,6 +208,12 @@ class UNet3D:
                     else:
                         grads[l.skip] = torch.empty(self._nvox(l.skip), l.cs, dtype=torch.float32, device=self.dev)
                     dS = grads[l.skip]
+                # scratch only where the gradient is split between two tensors or
+                # pooled; it goes straight into dA otherwise
+                dvin = dA
+                if l.up or l.skip:
+                    nvi = self._nvox(l.skip if l.up else l.src)
+                    dvin = torch.empty(nvi, l.ca + l.cs, dtype=torch.float32, device=self.dev)
             dW, dB = self._wviews(l, self.grad)
             wv, _ = self._wviews(l, self.wb)
             self.ctx.call("psc_conv3d_bwd", self._geom(l), gpu._p(a), gpu._p(s), gpu._p(wv), gpu._p(g),
