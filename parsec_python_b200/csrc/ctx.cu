@@ -27,8 +27,6 @@ extern "C" const char* psc_last_error(const psc_ctx* ctx) {
 // up to 16 blocks of destroyed contexts are kept for later ones, of the CUDA
 // context that pinned them only: cudaDeviceReset unpins and unmaps a device's
 // blocks, and what is pinned after it may lie at the same addresses.
-// A context that ended in an error may have a copy into its block in flight;
-// every call that succeeded has waited for its copies.
 constexpr size_t PIN_BYTES = 256 * sizeof(double);
 constexpr int PIN_KEEP = 16;
 struct PinBlock {
@@ -84,7 +82,7 @@ static void pin_give(psc_ctx* ctx) {
   double* p = ctx->host_scalars;
   ctx->host_scalars = nullptr;
   if (!p) return;
-  if (ctx->host_owner != 0 && ctx->last_error.empty()) {
+  if (ctx->host_owner != 0) {
     std::lock_guard<std::mutex> lk(g_pin_mu);
     if (g_pin_count < PIN_KEEP) {
       g_pin_free[g_pin_count++] = PinBlock{p, ctx->device, ctx->host_owner};
@@ -186,6 +184,16 @@ void psc_free_projectors(psc_ctx* ctx);
 
 extern "C" int psc_ctx_destroy(psc_ctx* ctx) {
   if (!ctx) return 0;
+  // The context's memory goes back to pools that do not know the streams it was
+  // used on (the device pool is ordered with the legacy stream alone), so
+  // whatever is still queued ends first.  (cudaFreeHost, where nothing is kept,
+  // waits in the same way.)
+  int dev = -1;
+  if (cudaGetDevice(&dev) == cudaSuccess) {
+    if (dev != ctx->device) cudaSetDevice(ctx->device);
+    cudaDeviceSynchronize();
+    if (dev != ctx->device) cudaSetDevice(dev);
+  }
   for (auto& s : ctx->species) free_species(s);
   psc_free_projectors(ctx);
   psc_dfree(ctx->pot64); psc_dfree(ctx->pot32); psc_dfree(ctx->cheb_coef); psc_dfree(ctx->red_partial);
