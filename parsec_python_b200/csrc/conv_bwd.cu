@@ -37,7 +37,7 @@
 //                channels at a time.
 //
 // One training step's backward on 82^3 voxels (19 G multiply-adds for each
-// product): weights 8.3 -> 0.76 ms, inputs 3.6 -> 0.92 ms against one thread
+// product): weights 8.3 -> 0.80 ms, inputs 3.6 -> 0.95 ms against one thread
 // per weight (two shared-memory loads per multiply-add) and one thread per
 // voxel on the CUDA cores.  (0.10 and 0.48 ms of
 // that were address arithmetic: a voxel's position is divided out once per

@@ -1,7 +1,8 @@
 // Persistent conjugate-gradient kernel for the Hartree solve
 // (Eigensolvers/pcg.py:7-85), one cooperative launch per solve.  Two forms:
-// the grid in boxes (k_cg_box, below) wherever a cut of it fits, up to about
-// 86^3, and in flat ranges (k_cg_persistent) on the sizes from there to 93^3.
+// the grid in boxes (k_cg_box, below) wherever a cut of it fits, for cubes up to
+// 84^3 (order 8, 148 SMs), and in flat ranges (k_cg_persistent) from there to
+// 93^3.
 //
 // The flat form.
 // The CG vectors of a whole grid fit in the shared memory of the GPU (a
@@ -220,12 +221,13 @@ k_cg_persistent(const double* __restrict__ rhs, double* __restrict__ xg, double*
 // PT points along z, its z neighbours in registers, and keeps p and Ap of the
 // run in registers for the whole solve (x, in shared memory, is touched once
 // per iteration; with it in registers the run's state spilled, and a release
-// waits for spilled stores too).  The halo points inside the grid
+// waits for spilled stores too; runs of more than 8 points still spill 88 bytes).  The halo points inside the grid
 // (an address and a slot each) are listed once; those outside stay zero.
-// 200 iterations at 78^3: 2420 -> 1950 us, at 52^3: 1620 -> 1280 (with grid_reduce
-// below).  Of an iteration's 9.8 and 6.4 us the two reductions with their
-// grid-wide visibility take 5.9; the rest is bound by shared-memory loads
-// (17 per point) and FP64 issue.
+// 200 iterations take 1913 us at 78^3 and 1307 at 52^3 (solves of 2460 and 1620 in
+// flat ranges, 1985 and 1370 now).  Of an iteration's 9.6 and 6.5 us the two
+// reductions with their grid-wide visibility take 5.9; the rest is bound by
+// shared-memory loads (17 per point) and FP64 issue.  (Counters: 7.3 warps
+// stalled at a barrier and 3.2 on shared memory per issue.)
 // ---------------------------------------------------------------------------
 constexpr int BOX_NT = 512;
 constexpr int BOX_PAD = 16;   // row pitch - box width (>= 2 R, a multiple of the 16 8-byte banks)
@@ -549,7 +551,7 @@ int psc_pcg_persistent(psc_ctx* ctx, const double* rhs, double* x, int maxit, do
   size_t smem = (5 * (size_t)chunk + 2 * (size_t)R * ctx->nx) * sizeof(double);
   int optin = 0;
   PSC_CUDA(ctx, cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-  // boxes where a cut fits (up to about 90^3), flat ranges on the few sizes above
+  // boxes where a cut fits, flat ranges above (cubes of 85^3 to 93^3 at order 8)
   BoxPlan plan;
   int pt = 0, threads = PNT;
   size_t box_smem = 0;

@@ -75,8 +75,10 @@ __global__ void k_sad(int nx, int ny, int nz, double h, double rad, int natoms, 
 //   - an atomic charge is skipped where its last interval is safely negative
 //     (it is clamped at zero there).
 // Every (atom, point) sum is taken in k_sad's order.  163 atoms on 90^3
-// points: 3685 -> 1186 us; the limit is now shared-memory gathers (about 20
-// per point and atom, three-way conflicts) and FP64 issue.
+// points: 3685 -> 1186 us; the limit is now the chain of dependent steps of a
+// look-up (3.4 warps wait for a fixed latency per issue, 54 % issue active) and
+// its shared-memory gathers (about 20 per point and atom, a quarter of their
+// wavefronts conflicts, pipe 64 % busy).
 constexpr int ST_NT = 320, ST_P = 4;          // threads per CTA, points per thread
 constexpr int ST_B0 = (127 - 7) << 6;         // first bucket: r = 2^-7
 constexpr int ST_NB = 14 << 6;                // up to r = 2^7

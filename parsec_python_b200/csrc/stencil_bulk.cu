@@ -16,6 +16,10 @@
 // thread before it arms the slot's barrier.
 //
 // H X at 61 x 55 x 67 with 31 columns: 124 -> 98 us, the step itself 101 -> 81.
+// What is left is the chain of a plane's edge tests, loads and adds in 16 warps
+// per SM and the unrolled loop's fetch: issue active 56 %, per issue 1.7 warps
+// wait for a fixed latency and 1.1 for instructions, the shared-memory pipe is
+// 43 % busy.
 // Points of a thread are 256 apart, so shared-memory and global accesses of a
 // warp are consecutive without any alignment.  Waits are bounded as in
 // stencil_tma.cu (status word 3).

@@ -35,8 +35,9 @@
 // only the potential, two planes ahead into registers instead saves a few
 // instructions more and loses it all: 1.5 to 7.6 warps stalled on the loads
 // per issue.  Under full HBM load two planes are not early enough.)
-// With this a step at 90^3, k = 307 takes 635 us in FP32 and 1203 in FP64 (709
-// and 1346 before), and 34.5 instead of 40.6 us at 52^3, k = 27.  The limit now is the
+// With this a step at 90^3, k = 307 takes 635 us in FP32 and 1204 in FP64 (709
+// and 1346 before; under the power cap of a long run FP64 takes 1265, 1358
+// before), and 34.5 instead of 40.6 us at 52^3, k = 27.  The limit now is the
 // shared-memory pipe, busy 77 % of the cycles: 24 neighbours of which the x and y
 // ones are loads.  (Giving a thread several rows, so that most y neighbours are
 // its own registers, cut the wavefronts by a fifth and was still slower: 1275 us

@@ -122,7 +122,7 @@ k_conv_fwd(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict_
 // input brick with its halo is staged once for all the taps.  The plain
 // kernel above fetches two weight vectors per input value for eight
 // multiply-adds and reads the input 27 times through L1 (852 us for the three
-// layers of a 90^3 pass); this one takes 456 us and is bound by the FP32 pipe.  Every output adds its terms in k_conv_fwd<8>'s order (32
+// layers of a 90^3 pass); this one takes 450 us and is bound by the FP32 pipe.  Every output adds its terms in k_conv_fwd<8>'s order (32
 // input channels at a time, taps, channels), so the results are the same
 // bits.  A tap outside the grid adds a zero product here, which an infinite or
 // NaN weight would turn into NaN: a thread that ends with a NaN takes its
@@ -442,7 +442,7 @@ extern "C" int psc_conv3d_fwd(psc_ctx* ctx, const int* geom, const void* A, cons
   // the tensor cores where a layer has 32 or more output channels; with 8 (N
   // padded to 16) half of every MMA is padding and the gather costs as much as
   // for 16, so the full-grid layers are faster on the CUDA cores (90^3: 40 -> 8
-  // channels 360 against 384 us, 8 -> 8 71 against 279).  Layers of stride 1 whose
+  // channels 366 against 384 us, 8 -> 8 71 against 279).  Layers of stride 1 whose
   // channels are no multiple of 16 take the eight-channel brick kernel, the
   // rest (16 channels, stride 2) the plain one, whose 27 reads of a voxel hit L1.
   if (ctx->conv_tc == 2 || (ctx->conv_tc == 1 && g.Cout >= 32))
